@@ -164,7 +164,10 @@ typedef struct psx_plan {
      returns at once).  0 = the default, 1 << 22 polls (about a second).  A small value
      lets a test make a wait run out without faulting the GPU. */
   int32_t wait_spins;
-  int32_t reserved0;        /* 0 */
+  /* Non-zero: the Tet4 sweeps without a tangent run in two launches (element tiles, then
+     node sums) on records of the whole mesh, without queue or waits; psx_work_bytes counts
+     those records.  The values are the queued kernels' bit for bit. */
+  int32_t two_pass;
 } psx_plan_t;
 
 /* n_pairs = (sum deg - N) / 2 and the pair_src length E * npe (npe - 1) / 2 (host). */

@@ -133,7 +133,7 @@ class PlanStruct(ctypes.Structure):
         ("n_gtasks_k", ctypes.c_int64),
         ("gtasks_k", ctypes.c_void_p),
         ("wait_spins", ctypes.c_int32),
-        ("reserved0", ctypes.c_int32),
+        ("two_pass", ctypes.c_int32),
     ]
 
 

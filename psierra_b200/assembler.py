@@ -109,15 +109,21 @@ class GPUAssembler:
                   ring_slack: int | None = None, lag_f: int | None = None, split: bool | None = None) -> None:
         """Launch shape of the persistent kernel (see ``MeshPattern.set_queue``)."""
         p = self.pattern
-        old = (p.lag, p.lag_f, p.ring_slack)
+        old = (p.lag, p.lag_f, p.ring_slack, p.two_pass)
         p.set_queue(lag=lag, blocks_per_sm=blocks_per_sm, ring_slack=ring_slack, lag_f=lag_f, split=split)
-        if (p.lag, p.lag_f, p.ring_slack) != old:
-            self._work.clear()  # the record ring is sized by the lag and the slack
+        if (p.lag, p.lag_f, p.ring_slack, p.two_pass) != old:
+            self._work.clear()  # the records are sized by the lag, the slack and the passes
+
+    def set_two_pass(self) -> None:
+        """Back to the two-pass sweeps after ``set_queue`` (see ``MeshPattern.two_pass``)."""
+        self.pattern.set_two_pass()
+        self._work.clear()
 
     def set_wait_limit(self, spins: int) -> None:
         """Polls after which a bounded wait of the persistent kernels gives up (0 = the
         default, about a second); see ``MeshPattern.set_wait_limit``."""
         self.pattern.set_wait_limit(spins)
+        self._work.clear()  # a limit selects the queued kernels, whose records are a ring
 
     def workspace(self, precision: str) -> torch.Tensor:
         w = self._work.get(precision)

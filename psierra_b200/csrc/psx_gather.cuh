@@ -773,7 +773,9 @@ inline int work_layout(const psx_plan_t* P, int precision, void* work, WorkLayou
   int32_t ring = 1;
   const int32_t lag = queue_k || P->lag_f <= 0 ? P->lag : P->lag_f;
   while (ring < W->span_g + lag + slack) ring <<= 1;
-  W->ring_g = ring < all ? ring : all;
+  // two-pass sweeps keep the records of the whole mesh
+  const bool whole = P->two_pass && P->npe == 4 && !queue_k;
+  W->ring_g = ring < all && !whole ? ring : all;
   W->ring_elems = (int64_t)W->ring_g * P->granule;
   const int sms = device_sm_count();
   if (sms <= 0) return PSX_ERR_CUDA;
@@ -788,7 +790,7 @@ inline int work_layout(const psx_plan_t* P, int precision, void* work, WorkLayou
   W->counter_bytes = (size_t)up(4 * (2 + 2 * (int64_t)P->n_granules));
   int64_t kbytes, fbytes;
   if (W->tiles) {
-    const int64_t ring_tiles = W->ring_elems / P->tile;
+    const int64_t ring_tiles = whole ? (P->n_elements + P->tile - 1) / P->tile : W->ring_elems / P->tile;
     // planar tile records (GatherArgs): 9 cap_p4 + 6 cap_n4 K values, 3 cap_n4 f doubles
     const int64_t cp4 = (P->tile_cap_pairs + 3) / 4 * 4, cn4 = (P->tile_cap_nodes + 3) / 4 * 4;
     kbytes = queue_k ? up(ring_tiles * (9 * cp4 + 6 * cn4) * kt) : 0;

@@ -29,9 +29,6 @@ namespace psx {
 namespace {
 
 constexpr int kThreads = 128;
-constexpr int kModeDR = 16;       // internal: PSX_KV with the fused dynamic-relaxation epilogue
-constexpr int kModeAdjoint = 64;  // internal: vector-Jacobian product of f_int
-constexpr int kModeEff = 128;     // internal: c_t K_T + c_m M + c_0 K_0 (dynamic effective tangent)
 #ifndef PSX_TET4_MIN_BLOCKS
 #define PSX_TET4_MIN_BLOCKS 3
 #endif
@@ -56,25 +53,6 @@ constexpr int kMinBlocks = PSX_TET4_MIN_BLOCKS;  // resident blocks per SM the r
 #ifndef PSX_TET4_MIN_BLOCKS_ADJ
 #define PSX_TET4_MIN_BLOCKS_ADJ 2
 #endif
-
-struct Tet4Args {
-  const int32_t* conn;
-  const double* X;
-  const double* U;
-  const double* Vv;  // vector of the matrix-free product (PSX_KV) / cotangent (adjoint)
-  double* dmu;       // adjoint: d(w.f)/d mu_e (E), or null
-  double* dkappa;    // adjoint: d(w.f)/d kappa_e (E), or null
-  const double* mu_e;
-  const double* kappa_e;
-  double mu0, kappa0, lam0;
-  Status* st;
-  // effective tangent (kModeEff): K_eff = c_t K_T + c_m M + c_0 K_0, M the consistent mass
-  // of density rho, K_0 the small-strain stiffness (lam0, mu0, or per element
-  // lambda = kappa_e - 2/3 mu_e, mu_e)
-  double c_t, c_m, c_0, rho;
-  // element records in the global ring (store_planes): the ring length (set by run_tet4)
-  int64_t plane = 0;
-};
 
 // Phase A: one element -> its record.  tet4_total_lagrangian.py:77-139 (and, with
 // PSX_LINEAR, tet4_base.py:129-136) in the closed form of psx_common.cuh.
@@ -119,18 +97,6 @@ __device__ __forceinline__ void put_diag(KT* __restrict__ krec, int o, const KT 
   }
 }
 
-// Explicitly rounded operations in the tangent's type (dmul / fmul etc. of psx_common.cuh).
-__device__ __forceinline__ double xmul(double a, double b) { return dmul(a, b); }
-__device__ __forceinline__ float xmul(float a, float b) { return fmul(a, b); }
-__device__ __forceinline__ double xadd(double a, double b) { return dadd(a, b); }
-__device__ __forceinline__ float xadd(float a, float b) { return fadd(a, b); }
-__device__ __forceinline__ double xfma(double a, double b, double c) { return dfma(a, b, c); }
-__device__ __forceinline__ float xfma(float a, float b, float c) { return ffma(a, b, c); }
-template <typename T>
-__device__ __forceinline__ T xdot3(T a0, T b0, T a1, T b1, T a2, T b2) {
-  return xfma(a0, b0, xfma(a1, b1, xmul(a2, b2)));
-}
-
 // `cn` = the element's connectivity (loaded by the caller, possibly ahead of time).
 template <typename KT, int MODE, bool KGLOBAL = true, bool FGLOBAL = true>
 __device__ __forceinline__ void tet4_element(const Tet4Args& A, int64_t e, const int4 cn, KT* __restrict__ krec,
@@ -167,8 +133,6 @@ __device__ __forceinline__ void tet4_element(const Tet4Args& A, int64_t e, const
   KT p[4][3], q[4][3];
   TangentCoef<KT> tc;
   KT gk[4][3];
-  // copies kept for the adjoint branch (dead code otherwise)
-  double ps_F[3][3], ps_Finv[3][3], ps_P[3][3], ps_lnJ = 0.0, Un_[4][3], l_[3][3];
 #pragma unroll
   for (int b = 0; b < 4; ++b)
 #pragma unroll
@@ -192,196 +156,35 @@ __device__ __forceinline__ void tet4_element(const Tet4Args& A, int64_t e, const
     PointState ps;
     neohookean_point(l, mu, kappa, ps);
     if (G.detD > 0.0 && ps.Jm1 <= -1.0) flag_bad_element(A.st, e, false);
-    if constexpr (kAdj) {
-#pragma unroll
-      for (int i = 0; i < 3; ++i)
-#pragma unroll
-        for (int j = 0; j < 3; ++j) {
-          ps_F[i][j] = ps.F[i][j];
-          ps_Finv[i][j] = ps.Finv[i][j];
-          ps_P[i][j] = ps.P[i][j];
-          l_[i][j] = l[i][j];
-        }
-      ps_lnJ = ps.lnJ;
-#pragma unroll
-      for (int b = 0; b < 4; ++b)
-#pragma unroll
-        for (int k = 0; k < 3; ++k) Un_[b][k] = Un[b][k];
-    }
     if constexpr (kWantF) {
       double fr[12];
-#pragma unroll
-      for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int i = 0; i < 3; ++i)
-          fr[3 * a + i] = dmul(G.V, ddot3(ps.P[i][0], G.g[a][0], ps.P[i][1], G.g[a][1], ps.P[i][2], G.g[a][2]));
+      tet4_force(ps, G, fr);
       store_f12<FGLOBAL>(frec, fr, A.plane);
     }
     if constexpr (kWantK || kKV) {
       tc = tangent_coef<KT>(ps, kappa, G.V);
-      KT Fi[3][3], Fm[3][3];
-#pragma unroll
-      for (int i = 0; i < 3; ++i)
-#pragma unroll
-        for (int j = 0; j < 3; ++j) {
-          Fi[i][j] = (KT)ps.Finv[i][j];
-          Fm[i][j] = (KT)ps.F[i][j];
-        }
-#pragma unroll
-      for (int b = 0; b < 4; ++b)
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-          p[b][k] = xdot3(Fi[0][k], gk[b][0], Fi[1][k], gk[b][1], Fi[2][k], gk[b][2]);
-          q[b][k] = xdot3(Fm[k][0], gk[b][0], Fm[k][1], gk[b][1], Fm[k][2], gk[b][2]);
-        }
+      tet4_pq<KT>(ps, gk, p, q);
     }
-  }
-  if constexpr (kKV) {
-    // y_a = sum_b K_ab v_b = alpha p_a + Pv h_a + beta (c q_a) + phi (sum_b (g_a.g_b) v_b)
-    // with alpha = sum_b w_b.v_b, beta = sum_b p_b.v_b, Pv = sum_b p_b v_b^T.
-    // L2 loads: in the fused dynamic-relaxation step the vector is updated in place later
-    // in the same launch (after every element reading a node has been evaluated).
-    double Vn[4][3];
-    {
-      const int ids[4] = {cn.x, cn.y, cn.z, cn.w};
+    if constexpr (kKV) {
+      // L2 loads: in the fused dynamic-relaxation step the vector is updated in place later
+      // in the same launch (after every element reading a node has been evaluated).
+      double Vn[4][3];
+      {
+        const int ids[4] = {cn.x, cn.y, cn.z, cn.w};
 #pragma unroll
-      for (int b = 0; b < 4; ++b)
+        for (int b = 0; b < 4; ++b)
 #pragma unroll
-        for (int k = 0; k < 3; ++k) Vn[b][k] = __ldcg(A.Vv + 3 * (int64_t)ids[b] + k);
-    }
-    KT vk[4][3];
-#pragma unroll
-    for (int b = 0; b < 4; ++b)
-#pragma unroll
-      for (int k = 0; k < 3; ++k) vk[b][k] = (KT)Vn[b][k];
-    KT alpha = 0, beta = 0, Pv[3][3], Gv[3][3];
-#pragma unroll
-    for (int k = 0; k < 3; ++k)
-#pragma unroll
-      for (int m = 0; m < 3; ++m) Pv[k][m] = Gv[k][m] = (KT)0;
-#pragma unroll
-    for (int b = 0; b < 4; ++b) {
-#pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        alpha = xfma(xfma(tc.A, p[b][k], xmul(tc.c, q[b][k])), vk[b][k], alpha);
-        beta = xfma(p[b][k], vk[b][k], beta);
-#pragma unroll
-        for (int m = 0; m < 3; ++m) {
-          Pv[k][m] = xfma(p[b][k], vk[b][m], Pv[k][m]);
-          Gv[k][m] = xfma(gk[b][k], vk[b][m], Gv[k][m]);
-        }
+          for (int k = 0; k < 3; ++k) Vn[b][k] = __ldcg(A.Vv + 3 * (int64_t)ids[b] + k);
       }
+      Tet4Sums<KT> S;
+      tet4_sums<KT>(tc, p, q, gk, Vn, S);
+      double yr[12];
+      if constexpr (kAdj)
+        tet4_vjp(A, e, true, ps, l, G, Un, Vn, tc, S, yr);
+      else
+        tet4_product<KT>(tc, p, q, gk, S, yr);
+      store_f12<FGLOBAL>(frec, yr);
     }
-    double yr[12];
-    if constexpr (!kAdj) {
-#pragma unroll
-      for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-          KT t = xfma(alpha, p[a][k], xmul(xmul(beta, tc.c), q[a][k]));
-#pragma unroll
-          for (int m = 0; m < 3; ++m)
-            t = xadd(t, xfma(Pv[k][m], xmul(tc.hb, p[a][m]), xmul(xmul(tc.phi, gk[a][m]), Gv[m][k])));
-          yr[3 * a + k] = (double)t;
-        }
-    } else {
-      // Vector-Jacobian product of w.f_e with f_e,a = V P g_a (the adjoint of
-      // tet4_total_lagrangian.py:136-137 w.r.t. X, mu, kappa).  L_w = sum_b w_b g_b^T,
-      // VM = V dP/dF[L_w] = alpha F^-T + hb Pv F^-T + beta c F + phi Gv^T.
-      double Fi[3][3], Fm[3][3], VM[3][3], Lw[3][3];
-#pragma unroll
-      for (int i = 0; i < 3; ++i)
-#pragma unroll
-        for (int j = 0; j < 3; ++j) {
-          Fi[i][j] = (double)ps_Finv[i][j];
-          Fm[i][j] = (double)ps_F[i][j];
-          Lw[i][j] = 0.0;
-        }
-#pragma unroll
-      for (int b = 0; b < 4; ++b)
-#pragma unroll
-        for (int i = 0; i < 3; ++i)
-#pragma unroll
-          for (int j = 0; j < 3; ++j) Lw[i][j] += Vn[b][i] * G.g[b][j];
-#pragma unroll
-      for (int k = 0; k < 3; ++k)
-#pragma unroll
-        for (int m = 0; m < 3; ++m) {
-          // (F^-T)[k][m] = Finv[m][k]
-          double t = (double)alpha * Fi[m][k] + (double)beta * (double)tc.c * Fm[k][m] + (double)tc.phi * (double)Gv[m][k];
-#pragma unroll
-          for (int j = 0; j < 3; ++j) t += (double)Pv[k][j] * (double)tc.hb * Fi[m][j];
-          VM[k][m] = t;
-        }
-      // h_b = VM^T u_b + V P^T w_b  (vectors conjugate to dg_b)
-      double h[4][3];
-#pragma unroll
-      for (int b = 0; b < 4; ++b)
-#pragma unroll
-        for (int j = 0; j < 3; ++j) {
-          double t = 0.0;
-#pragma unroll
-          for (int i = 0; i < 3; ++i) t += VM[i][j] * Un_[b][i] + G.V * ps_P[i][j] * Vn[b][i];
-          h[b][j] = t;
-        }
-      double PL = 0.0;
-#pragma unroll
-      for (int i = 0; i < 3; ++i)
-#pragma unroll
-        for (int j = 0; j < 3; ++j) PL += ps_P[i][j] * Lw[i][j];
-      // dL/dD = PL V G^T - G^T Hm G^T with G = D^-1 (rows g_1..g_3), Hm rows h_b - h_0
-      double Gm[3][3], Hm[3][3], T1[3][3], Z[3][3];
-#pragma unroll
-      for (int r = 0; r < 3; ++r)
-#pragma unroll
-        for (int j = 0; j < 3; ++j) {
-          Gm[r][j] = G.g[r + 1][j];
-          Hm[r][j] = h[r + 1][j] - h[0][j];
-        }
-#pragma unroll
-      for (int i = 0; i < 3; ++i)  // T1 = G^T Hm
-#pragma unroll
-        for (int j = 0; j < 3; ++j) T1[i][j] = Gm[0][i] * Hm[0][j] + Gm[1][i] * Hm[1][j] + Gm[2][i] * Hm[2][j];
-#pragma unroll
-      for (int i = 0; i < 3; ++i)
-#pragma unroll
-        for (int j = 0; j < 3; ++j)
-          Z[i][j] = PL * G.V * Gm[j][i] - (T1[i][0] * Gm[j][0] + T1[i][1] * Gm[j][1] + T1[i][2] * Gm[j][2]);
-      // D[i][j] = X_{j+1}[i] - X_0[i]
-#pragma unroll
-      for (int i = 0; i < 3; ++i) {
-        yr[i] = -(Z[i][0] + Z[i][1] + Z[i][2]);
-#pragma unroll
-        for (int j = 0; j < 3; ++j) yr[3 * (j + 1) + i] = Z[i][j];
-      }
-      // parameter gradients: dP/dmu = 2 J^-2/3 F^-T dev E, dP/dkappa = ln J F^-T
-      if (A.dmu || A.dkappa) {
-        double E[3][3], trE = 0.0;
-#pragma unroll
-        for (int i = 0; i < 3; ++i)
-#pragma unroll
-          for (int j = 0; j < 3; ++j) {
-            const double ltl = l_[0][i] * l_[0][j] + l_[1][i] * l_[1][j] + l_[2][i] * l_[2][j];
-            E[i][j] = 0.5 * (l_[i][j] + l_[j][i] + ltl);
-          }
-        trE = E[0][0] + E[1][1] + E[2][2];
-        const double jm23 = exp((-2.0 / 3.0) * ps_lnJ);
-        double FTL = 0.0, FDL = 0.0;
-#pragma unroll
-        for (int i = 0; i < 3; ++i)
-#pragma unroll
-          for (int j = 0; j < 3; ++j) {
-            FTL += Fi[j][i] * Lw[i][j];
-            double fd = 0.0;  // (F^-T dev E)[i][j]
-#pragma unroll
-            for (int k = 0; k < 3; ++k) fd += Fi[k][i] * (E[k][j] - (k == j ? trE / 3.0 : 0.0));
-            FDL += fd * Lw[i][j];
-          }
-        if (A.dmu) A.dmu[e] = G.V * 2.0 * jm23 * FDL;
-        if (A.dkappa) A.dkappa[e] = G.V * ps_lnJ * FTL;
-      }
-    }
-    store_f12<FGLOBAL>(frec, yr);
   }
   if constexpr (kWantK) {
     // K_ab[k][m] = p_a,k w_b,m + p_b,k h_a,m + y_a,k p_b,m + s_ab d_km
@@ -757,6 +560,72 @@ tet4_split_kernel(Tet4Args A, GatherArgs g, QueueArgs Q, const int4* __restrict_
   }
 }
 
+// ---- two-pass sweeps ------------------------------------------------------------------
+// The sweeps without a tangent (f, K.v, dynamic relaxation, adjoint) in two launches: one
+// warp per element tile writes its tile record, then one thread per node sums the records.
+// Same element code, records and association as the queue, so the same bits; but no
+// claims, waits or completion counts, warps that hold only what an element tile needs
+// (16-20 per SM), and gathers at full occupancy, 12 blocks of them behind each SM's loads
+// instead of a turn in the queue.  The records of the whole mesh are kept (22 bytes per
+// element, in L2 up to about 5M elements).  Measured, queue -> two passes, us:
+//   elements    f              K.v FP32        K.v FP64
+//     384,000    71 ->  28      69 ->  33       80 ->  35
+//   1,053,696   106 ->  64     120 ->  83      121 ->  84
+//   3,072,000   272 -> 174     297 -> 231      320 -> 231
+// What bounds them now is the latency of the FP64 element chain (47% issue; the FP64 pipe
+// alone would take 21 us at 1.05M elements).  Passing over the mesh in pieces, so that the
+// records stay in L2, only adds launches (1.05M elements, 16 pieces: f 104 us).
+template <typename KT, int MODE>
+__global__ void __launch_bounds__(kThreads, min_blocks<KT, MODE>())
+tet4_tiles_kernel(Tet4Args A, GatherArgs g, int64_t n_elements, double* __restrict__ frec) {
+  using S = Tet4Smem<KT, MODE>;
+  static_assert(S::kTiles && !S::kWantK, "tile records of a sweep without a tangent");
+  const int lane = threadIdx.x & 31;
+  extern __shared__ __align__(16) unsigned char s_stage[];
+  unsigned char* my_stage = s_stage + (threadIdx.x >> 5) * S::kWarpBytes;
+  double* fst = reinterpret_cast<double*>(my_stage);
+  unsigned char* lst = my_stage + sizeof(double) * S::kFDoubles;
+  const int64_t t = blockIdx.x * (int64_t)(kThreads / 32) + (threadIdx.x >> 5);
+  const int64_t e0 = t * g.tile;
+  if (e0 >= n_elements) return;
+  tile_meta_prefetch<false>(g, t, lst);
+  const int64_t e = e0 + lane;
+  if (lane < g.tile && e < n_elements)
+    tet4_element<KT, MODE, false, false>(A, e, __ldg(reinterpret_cast<const int4*>(A.conn) + e), nullptr,
+                                         fst + kFStride * lane);
+  cp_async_wait_all();
+  __syncwarp();
+  tile_reduce<false, true>(g, t, lst, nullptr, fst, nullptr, frec);
+}
+
+constexpr int kItemThreads = 128;
+template <int MODE>
+__global__ void __launch_bounds__(kItemThreads)
+tet4_nodes_kernel(GatherArgs g, int32_t n_nodes, const double* __restrict__ frec, double* __restrict__ f_out, DRArgs dr) {
+  const int32_t n = blockIdx.x * kItemThreads + threadIdx.x;
+  if (n < n_nodes)
+    gather_node<double, 4, false, true, (MODE & kModeDR) != 0, true>(g, node_head<true>(g, n), nullptr, frec, nullptr,
+                                                                     f_out, &dr);
+}
+
+template <typename KT, int MODE>
+int run_two_pass(const psx_plan_t* P, const Tet4Args& A, const WorkLayout& W, double* f_out, cudaStream_t stream,
+                 const DRArgs& dr) {
+  using S = Tet4Smem<KT, MODE>;
+  const GatherArgs g = gather_args(P, W.ring_elems);
+  if (!W.tiles || P->tile > 32 || g.meta_stride > kMetaBytes || P->n_nodes > 0x7fffffff) return PSX_ERR_ARG;
+  const size_t smem = (kThreads / 32) * S::kWarpBytes;
+  static unsigned long long s_smem_set = 0;
+  if (set_dynamic_smem_once(tet4_tiles_kernel<KT, MODE>, (int)smem, &s_smem_set) != cudaSuccess) return PSX_ERR_CUDA;
+  const int64_t tiles = (P->n_elements + P->tile - 1) / P->tile, per_block = kThreads / 32;
+  tet4_tiles_kernel<KT, MODE><<<(unsigned)((tiles + per_block - 1) / per_block), kThreads, smem, stream>>>(
+      A, g, P->n_elements, W.frec);
+  tet4_nodes_kernel<MODE><<<(unsigned)((P->n_nodes + kItemThreads - 1) / kItemThreads), kItemThreads, 0, stream>>>(
+      g, (int32_t)P->n_nodes, W.frec, f_out, dr);
+  PSX_CUDA_CHECK_LAUNCH();
+  return PSX_OK;
+}
+
 // The split kernel is usable when its compiled register count is the one its
 // setmaxnreg split is computed for (checked once per process: the count is a property
 // of the compiled kernel).
@@ -797,6 +666,10 @@ int run_tet4(const psx_plan_t* P, const Tet4Args& A, const WorkLayout& W, KT* k_
              cudaStream_t stream, const DRArgs& dr = DRArgs{}) {
   constexpr bool kWantK =
       (MODE & (PSX_WANT_K | PSX_LINEAR | PSX_MASS)) != 0 && (MODE & (PSX_KV | kModeAdjoint)) == 0;
+  // every sweep without a tangent is faster in two passes (tet4_tiles_kernel), at all sizes
+  if constexpr (!kWantK) {
+    if (P->two_pass) return run_two_pass<KT, MODE>(P, A, W, f_out, stream, dr);
+  }
   const GatherArgs g = gather_args(P, W.ring_elems);
   const QueueArgs Q = queue_args(P, W, kWantK);
   using S = Tet4Smem<KT, MODE>;

@@ -53,6 +53,7 @@ class MeshPattern:
         self._dev: dict | None = None
         self._blocks: tuple | None = None
         self._plan_host: dict | None = None
+        self.queued_f = False  # a lag of the f / K.v queue was chosen (set_queue)
         self.granule, self.tile, self.tile_items, self.lag, self.lag_f, self.ring_slack = self.QUEUE[npe]
         self.blocks_per_sm = 0
         self.wait_spins = 0  # polls of one bounded wait in the persistent kernels (0 = about a second)
@@ -208,8 +209,21 @@ class MeshPattern:
     def _apply_split(self, d: dict) -> None:
         st = d["plan"]
         on = self.split and d.get("n_gtasks_k", 0) > 0
+        st.two_pass = int(self.two_pass)
         st.n_gtasks_k = d["n_gtasks_k"] if on else 0
         st.gtasks_k = d["gtasks_k"].data_ptr() if on else None
+
+    @property
+    def two_pass(self) -> bool:
+        """Whether the Tet4 sweeps without a tangent run in two passes: by default, until a
+        lag of their queue is chosen (``set_queue(lag_f=...)``) or its waits are limited."""
+        return self.npe == 4 and not self.queued_f and self.wait_spins == 0
+
+    def set_two_pass(self) -> None:
+        """Back to the two-pass sweeps after ``set_queue``; a workspace must be re-queried."""
+        self.queued_f = False
+        if self._dev is not None:
+            self._apply_split(self._dev)
 
     def set_wait_limit(self, spins: int) -> None:
         """Polls after which a bounded wait of the persistent kernels gives up (0 = the
@@ -220,6 +234,7 @@ class MeshPattern:
         self.wait_spins = int(spins)
         if self._dev is not None:
             self._dev["plan"].wait_spins = self.wait_spins
+            self._apply_split(self._dev)
 
     def set_queue(self, lag: int | None = None, blocks_per_sm: int | None = None,
                   ring_slack: int | None = None, lag_f: int | None = None, split: bool | None = None) -> None:
@@ -228,7 +243,8 @@ class MeshPattern:
         span + lag; 0 = the minimum, 6) and whether Tet4 FP32 tangent sweeps run the
         warp-specialised kernel (``split``; the mixed kernel otherwise).
 
-        Rebuilds the task queues when a lag changes; a workspace sized for the old values
+        With ``lag_f``, the sweeps without a tangent run the queued kernel instead of two
+        passes (``set_two_pass`` goes back).  Rebuilds the task queues when a lag changes; a workspace sized for the old values
         must be re-queried (``psx_work_bytes``) afterwards.
         """
         rebuild = (lag is not None and int(lag) != self.lag) or (lag_f is not None and int(lag_f) != self.lag_f)
@@ -239,6 +255,7 @@ class MeshPattern:
             self.lag = int(lag)
         if lag_f is not None:
             self.lag_f = int(lag_f)
+            self.queued_f = True
         if blocks_per_sm is not None:
             self.blocks_per_sm = int(blocks_per_sm)
         if ring_slack is not None:

@@ -1,0 +1,100 @@
+"""Tet4 sweeps in two passes against the queued kernels (GPU).
+
+Same element code, tile records and association: f, K.v, dynamic relaxation and the adjoint
+must be equal bit for bit.  Meshes at the edges of the tiles: one element, a last tile of
+one element, ragged boxes, shuffled numbering (wide spans, many nodes per tile), disjoint
+unions, a mesh of many granules.
+"""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+import torch
+
+from psierra_b200 import meshgen
+from psierra_b200.assembler import GPUAssembler
+from psierra_b200.material import NeoHookeanField
+
+pytestmark = pytest.mark.gpu
+DEV = torch.device("cuda")
+
+
+def _shuffled(mesh, seed):
+    rng = np.random.default_rng(seed)
+    new = rng.permutation(mesh.n_nodes)
+    nodes = np.empty_like(mesh.nodes)
+    nodes[new] = mesh.nodes
+    return meshgen.TetMesh(nodes, new[mesh.elements][rng.permutation(mesh.n_elements)])
+
+
+def _cut(mesh, n):
+    el = mesh.elements[:n]
+    used, local = np.unique(el, return_inverse=True)
+    return meshgen.TetMesh(mesh.nodes[used], local.reshape(el.shape))
+
+
+MESHES = {
+    "one element": lambda: meshgen.TetMesh(np.vstack([np.zeros(3), np.eye(3)]), np.array([[0, 1, 2, 3]])),
+    "33 elements": lambda: _cut(meshgen.box_tet4(1.0, 1.0, 1.0, 2, 2, 2), 33),
+    "ragged box": lambda: meshgen.box_tet4(1.0, 0.3, 0.5, 7, 3, 5),
+    "shuffled box": lambda: _shuffled(meshgen.box_tet4(1.0, 1.0, 1.0, 11, 12, 13), 3),
+    "uneven beams": lambda: meshgen.concat_meshes([c.mesh for c in meshgen.beam_batch(n=12, target_tets=60000, seed=3)])[0],
+    "cube 44": lambda: meshgen.box_tet4(1.0, 1.0, 1.0, 44, 44, 44),
+}
+
+
+def _pair(mesh, precision):
+    mu = np.random.default_rng(4).uniform(1e3, 5e3, mesh.n_elements)
+    field = NeoHookeanField(mu, 20.0 * mu, mass_density=900.0)
+    a, b = (GPUAssembler(mesh.nodes, mesh.elements, field, precision=precision) for _ in range(2))
+    b.set_queue(lag_f=b.pattern.lag_f)
+    assert a.dev["plan"].two_pass == 1 and b.dev["plan"].two_pass == 0
+    X = mesh.nodes
+    ext = float(np.ptp(X, axis=0).max())
+    u = 0.03 * (X[:, [1, 2, 0]] - X.mean(axis=0)) + 0.002 * ext * np.sin(6.0 * X / ext)
+    v = np.random.default_rng(5).normal(size=3 * mesh.n_nodes)
+    return a, b, torch.from_numpy(u.reshape(-1)).to(DEV), torch.from_numpy(v).to(DEV)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32-mixed"])
+@pytest.mark.parametrize("name", list(MESHES))
+def test_two_pass_sweeps_equal_the_queued_kernels(name, precision):
+    a, b, u, v = _pair(MESHES[name](), precision)
+
+    def sweeps(s):
+        yield "f", s.assemble(u, want_k=False)[0]
+        yield "K.v", s.kv(u, v)
+        yield from zip(("X", "mu", "kappa"), s.adjoint(u, v))
+        x, vel, r = torch.zeros_like(v), torch.zeros_like(v), torch.empty_like(v)
+        for _ in range(3):
+            s.dr_step(u, v, torch.full_like(v, 1e-6), x, vel, 0.9, 1.9, 1.0, r_out=r)
+        yield from (("x", x), ("vel", vel), ("r", r))
+
+    for (what, x), (_, y) in zip(sweeps(a), sweeps(b)):
+        assert torch.equal(x, y), what
+    assert a.status_counts() == (0, 0, -1, 0)
+
+
+def test_workspace_follows_the_way_the_sweeps_run():
+    a, b, u, v = _pair(MESHES["cube 44"](), "fp64")
+    y = a.kv(u, v).clone()
+    a.set_queue(lag_f=2, ring_slack=6)
+    assert torch.equal(a.kv(u, v), y)
+    a.set_two_pass()
+    assert torch.equal(a.kv(u, v), y)
+    a.set_wait_limit(1 << 22)
+    assert a.dev["plan"].two_pass == 0 and torch.equal(a.kv(u, v), y)
+
+
+def test_captured_in_a_graph():
+    a, b, u, v = _pair(MESHES["ragged box"](), "fp64")
+    y = b.kv(u, v)
+    out = torch.empty_like(y)
+    a.kv(u, v, y_out=out, check_status=False)
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        a.kv(u, v, y_out=out, check_status=False)
+    out.zero_()
+    g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out, y)
