@@ -4,7 +4,7 @@ Mirrors ``HyperReducedECSWModel.evaluate_forces_and_stiffness`` (psierra
 ``hyperreduction/model.py:254-318``): only the elements of the reduced integration domain
 (RID) are evaluated, each at ``u_e = Phi_e u_r`` with its cubature weight, and projected
 onto the modal basis.  ``ECSWEvaluator`` caches the RID's reference coordinates, modal
-sub-bases and weights on the device once (``model.py:181-206``); one evaluation is two
+sub-bases and weights on the device once (``model.py:181-206``); one evaluation is three
 kernel launches (``psx_ecsw_evaluate``).
 """
 from __future__ import annotations
