@@ -549,6 +549,8 @@ int layout(int64_t n, int precond, void* work, PcgWork* w, int64_t* bytes) {
   return PSX_OK;
 }
 
+#include "psx_pcg_resident.cuh"
+
 template <typename VT, bool BLOCK, bool NODAL>
 int run_pcg(int64_t n, const int32_t* indptr, const int32_t* indices, const VT* vals, const double* b, double* x,
             double rtol, double atol, int32_t maxiter, const PcgWork& w, Status* st, cudaStream_t s,
@@ -556,6 +558,9 @@ int run_pcg(int64_t n, const int32_t* indptr, const int32_t* indices, const VT* 
   const int grid_vec = (int)std::min<int64_t>(kGridMax, (n + kBlock - 1) / kBlock);
   const int grid_row = NODAL ? (int)std::min<int64_t>(kGridMax, (n / 3 + kBlock / kNodeLanes - 1) / (kBlock / kNodeLanes))
                              : (int)std::min<int64_t>(kGridMax, (n + kBlock / kRowLanes - 1) / (kBlock / kRowLanes));
+  // systems whose state fits the shared memory of the GPU run in one launch
+  const int one = run_pcg_resident<VT, BLOCK, NODAL>(n, indptr, indices, vals, b, x, rtol, atol, maxiter, w, st, s, identity);
+  if (one != 0) return one > 0 ? PSX_OK : PSX_ERR_CUDA;
   if (cudaMemsetAsync(w.s, 0, sizeof(PcgScalars), s) != cudaSuccess) return PSX_ERR_CUDA;
   if (BLOCK)
     bjacobi_setup<<<grid_vec, kBlock, 0, s>>>(n / 3, indptr, indices, vals, sizeof(VT) == 4, w.minv, w.s);
