@@ -187,6 +187,23 @@ __device__ __forceinline__ void st_ring(double* q, double v) {
   asm volatile("st.global.L2::cache_hint.f64 [%0], %1, %2;" ::"l"(q), "d"(v), "l"(l2_keep_policy()) : "memory");
 }
 
+// Four doubles at a 32-byte aligned address in one load instruction (256 bits, sm_100).  A
+// warp's gathered loads cost one L1 pass per line and instruction, so a padded triple in one
+// load costs a third of three scalar ones.
+struct Quad {
+  double x, y, z, w;
+};
+__device__ __forceinline__ Quad ld_quad_nc(const double* p) {  // memory no thread of the launch writes
+  Quad q;
+  asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(q.x), "=d"(q.y), "=d"(q.z), "=d"(q.w) : "l"(p));
+  return q;
+}
+__device__ __forceinline__ Quad ld_quad(const double* p) {
+  Quad q;
+  asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(q.x), "=d"(q.y), "=d"(q.z), "=d"(q.w) : "l"(p));
+  return q;
+}
+
 // Three consecutive CSR values at p (aligned to the value size) in two streaming stores:
 // the two-value half that is aligned to twice the value size and the remaining value,
 // chosen by predicates so that the lanes of a warp do not diverge.  Each pair block then

@@ -17,14 +17,18 @@
 // C^-1 (x) I terms of the NeoHookean tangent drop out, and the C^-1 scalings of C_bar
 // cancel r^4.  The volumetric "div_e" rows (B_0 + B_1 + B_2) are q_b.
 //
-// Kernels (one thread per element, node, one-ring entry or two-ring block; every sum in
-// the reference's order, ascending element / ascending patch node):
+// Kernels (one thread per element, node, one-ring entry or two-ring block; every sum in a
+// fixed order, the reference's ascending element / patch node but for the longest lists,
+// which a warp adds as a tree).  Measured on 162,000 elements, us (before): 11 (16), 9 (9),
+// 30 (51), 75 (122), 111 (154), 76 (96).  What bounds them: the volumetric pass its
+// instructions and gathered loads, the element pass 8 warps per SM at 248 registers, the
+// gather the latency of its records.
 //   fbar_pre     V_e, J_e, q_e (and the inversion status)
 //   fbar_nodes   v0_a, J_node_a
 //   fbar_patch   g_a[b] = sum_{e in E_a, b in e} (V_e J_e / (4 v0_a)) q_e,b
 //   fbar_element element record: 6 pair blocks, 4 diagonal blocks, 12 forces
-//   fbar_gather  one-ring blocks and f (fixed-order sums of the records)
-//   fbar_vol     two-ring blocks += sum_a kappa v0_a g_a[b] g_a[c]^T
+//   fbar_vol     two-ring blocks = sum_a kappa v0_a g_a[b] g_a[c]^T
+//   fbar_gather  one-ring blocks += and f = fixed-order sums of the records
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -37,7 +41,10 @@ namespace psx {
 namespace {
 
 constexpr int kFbThreads = 128;
-constexpr int kFbRec = 6 * 9 + 4 * 6 + 12;  // doubles per element record
+// Element record: 6 pair blocks (9 values in 10), 4 diagonal blocks (6), 4 forces (3 in 4),
+// each a whole number of 16-byte loads.  (Blocks padded for 32-byte loads made the records a
+// fifth larger: element pass 109 instead of 74 us on 162,000 elements, gather no faster.)
+constexpr int kFbPair = 10, kFbDiag = 6 * kFbPair, kFbForce = kFbDiag + 4 * 6, kFbRec = kFbForce + 4 * 4;
 
 struct FbarArgs {
   const int32_t* conn;      // E x 4
@@ -53,11 +60,11 @@ struct FbarArgs {
   const double* jbar_in;    // optional per-element J_bar (overrides the nodal average)
   double* V;                // E
   double* J;                // E
-  double* q;                // 12 E
+  double* q;                // 16 E: (V_e J_e / 4) q_e,b, four doubles per node
   double* v0;               // N
   double* Jn;               // N
   double* Jbar;             // E (output: the J_bar used)
-  double* g;                // 3 x one-ring entries
+  double* g;                // 4 x one-ring entries: g_a[b], kappa v0_a
   double* rec;              // kFbRec x E
   Status* st;
   int64_t E, N;
@@ -101,23 +108,76 @@ __device__ __forceinline__ void fb_F(const double Un[4][3], const double g[4][3]
     }
 }
 
+// Copy a block's records (n x len doubles, staged in shared memory with `stride` doubles per
+// record) to consecutive global memory, whole lines at a time.  A thread storing its own
+// record wrote eight bytes of 32 sectors per instruction: the element pass took 122 us on
+// 162,000 elements, now 75 (22.5M sector writes, now 6.1M).
+// `at(j)`: place of value j in the record of LEN doubles.
+template <int VALS, int STRIDE, int LEN, typename At>
+__device__ __forceinline__ void fb_copy_records(double* __restrict__ out, const double* s, int n, At at) {
+  for (int k = threadIdx.x; k < n * VALS; k += blockDim.x) {
+    const int r = k / VALS, j = k - r * VALS;
+    out[r * LEN + at(j)] = s[r * STRIDE + j];
+  }
+}
+
+// The node of entry t0 + lane for the kernels with one thread per entry of ptr's runs: the
+// warp finds the node of t0 by a 32-way search (three dependent loads for 30,000 nodes; a
+// binary search per thread took fifteen), then the lanes step over the run ends among their
+// 32 entries.  Runs of unused nodes may be empty.
+__device__ __forceinline__ int64_t fb_node_of(const int32_t* __restrict__ ptr, int64_t N, int64_t t0, int lane) {
+  int64_t lo = 0, hi = N;  // ptr[lo] <= t0 < ptr[hi]
+  while (hi - lo > 1) {
+    const int64_t step = (hi - lo + 31) / 32;
+    const int64_t at = lo + step * (lane + 1);
+    const unsigned m = __ballot_sync(0xffffffffu, at < hi && __ldg(ptr + at) <= t0);
+    const int c = __popc(m);  // the true lanes are the first ones
+    hi = min(hi, lo + step * (c + 1));
+    lo += step * c;
+  }
+  int64_t node = lo;
+  for (int64_t k = lo + 1; k < N; ++k) {  // the same for all lanes: runs that start inside the warp's entries
+    const int32_t p = __ldg(ptr + k);
+    if (p >= t0 + 32) break;
+    if (p <= t0 + lane) node = k;
+  }
+  return node;
+}
+// Entries with more terms than this are summed by the whole warp, a term per lane (a node's
+// entry with itself has 15 or 24, most have one to eight); the others by their own lane.
+constexpr int kFbLong = 8;
+__device__ __forceinline__ double fb_warp_sum(double v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
 __global__ void __launch_bounds__(kFbThreads) fbar_pre(FbarArgs A) {
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < A.E; e += (int64_t)gridDim.x * blockDim.x) {
-    const int4 cn = reinterpret_cast<const int4*>(A.conn)[e];
-    double Xn[4][3], Un[4][3], g[4][3], F[3][3], detD;
-    fb_nodes(A.X, cn, Xn);
-    fb_nodes(A.U, cn, Un);
-    const double V = fb_geometry(Xn, g, detD);
-    if (!(detD > 0.0)) flag_bad_element(A.st, e, true);
-    fb_F(Un, g, F);
-    const double J = det3(F);
-    if (detD > 0.0 && !(J > 0.0)) flag_bad_element(A.st, e, false);
-    A.V[e] = V;
-    A.J[e] = J;
+  __shared__ double s_q[kFbThreads * 13];
+  for (int64_t e0 = blockIdx.x * (int64_t)kFbThreads; e0 < A.E; e0 += (int64_t)gridDim.x * kFbThreads) {
+    const int64_t e = e0 + threadIdx.x;
+    __syncthreads();
+    if (e < A.E) {
+      const int4 cn = reinterpret_cast<const int4*>(A.conn)[e];
+      double Xn[4][3], Un[4][3], g[4][3], F[3][3], detD;
+      fb_nodes(A.X, cn, Xn);
+      fb_nodes(A.U, cn, Un);
+      const double V = fb_geometry(Xn, g, detD);
+      if (!(detD > 0.0)) flag_bad_element(A.st, e, true);
+      fb_F(Un, g, F);
+      const double J = det3(F);
+      if (detD > 0.0 && !(J > 0.0)) flag_bad_element(A.st, e, false);
+      A.V[e] = V;
+      A.J[e] = J;
 #pragma unroll
-    for (int b = 0; b < 4; ++b)
+      for (int b = 0; b < 4; ++b)
 #pragma unroll
-      for (int k = 0; k < 3; ++k) A.q[12 * e + 3 * b + k] = F[k][0] * g[b][0] + F[k][1] * g[b][1] + F[k][2] * g[b][2];
+        for (int k = 0; k < 3; ++k)
+            s_q[13 * threadIdx.x + 3 * b + k] = 0.25 * V * J * (F[k][0] * g[b][0] + F[k][1] * g[b][1] + F[k][2] * g[b][2]);
+    }
+    __syncthreads();
+    fb_copy_records<12, 13, 16>(A.q + 16 * e0, s_q, (int)min((int64_t)kFbThreads, A.E - e0),
+                                [](int j) { return j + j / 3; });
   }
 }
 
@@ -136,40 +196,58 @@ __global__ void __launch_bounds__(kFbThreads) fbar_nodes(FbarArgs A) {
   }
 }
 
-// g_a[b] for every one-ring entry (a, b): thread per node a
-// One thread per one-ring entry t (node a and its neighbour; a found by a binary search
-// of nbr_ptr), so that a warp writes consecutive entries.
+// g_a[b] for every one-ring entry t (node a and its neighbour b), one thread per entry.
 __global__ void __launch_bounds__(kFbThreads) fbar_patch(FbarArgs A) {
-  const int64_t n1 = A.nbr_ptr[A.N];
-  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n1; t += (int64_t)gridDim.x * blockDim.x) {
-    int64_t lo = 0, hi = A.N;  // nbr_ptr[lo] <= t < nbr_ptr[hi]
-    while (hi - lo > 1) {
-      const int64_t mid = (lo + hi) / 2;
-      if (A.nbr_ptr[mid] <= t)
-        lo = mid;
-      else
-        hi = mid;
+  const int lane = threadIdx.x & 31;
+  const int64_t n1 = __ldg(A.nbr_ptr + A.N);
+  for (int64_t t0 = blockIdx.x * (int64_t)kFbThreads + (threadIdx.x & ~31); t0 < n1; t0 += (int64_t)gridDim.x * kFbThreads) {
+    const int64_t t = t0 + lane;
+    const int32_t s0 = __ldg(A.blk_ptr + min(t, n1)), s1 = __ldg(A.blk_ptr + min(t + 1, n1));
+    const double v0 = A.v0[fb_node_of(A.nbr_ptr, A.N, t0, lane)];
+    double g[3] = {0.0, 0.0, 0.0};
+    auto term = [&](int32_t s) {
+      const int32_t code = __ldg(A.blk_src + s);
+      return ld_quad_nc(A.q + 16 * (int64_t)(code >> 4) + 4 * (code & 3));
+    };
+    if (s1 - s0 <= kFbLong) {
+#pragma unroll 4
+      for (int32_t s = s0; s < s1; ++s) {
+        const Quad x = term(s);
+        g[0] += x.x;
+        g[1] += x.y;
+        g[2] += x.z;
+      }
     }
-    const double v0 = A.v0[lo];
-    double g0 = 0.0, g1 = 0.0, g2 = 0.0;
-    for (int32_t s = A.blk_ptr[t]; s < A.blk_ptr[t + 1]; ++s) {
-      const int32_t code = A.blk_src[s];
-      const int32_t lb = code & 3;
-      const int64_t e = code >> 4;
-      const double w = 0.25 * A.V[e] * A.J[e] / v0;
-      const double* qe = A.q + 12 * e + 3 * lb;
-      g0 += w * qe[0];
-      g1 += w * qe[1];
-      g2 += w * qe[2];
+    for (unsigned m = __ballot_sync(0xffffffffu, s1 - s0 > kFbLong); m; m &= m - 1) {
+      const int k = __ffs(m) - 1;
+      const int32_t a0 = __shfl_sync(0xffffffffu, s0, k), a1 = __shfl_sync(0xffffffffu, s1, k);
+      double h[3] = {0.0, 0.0, 0.0};
+      for (int32_t s = a0 + lane; s < a1; s += 32) {
+        const Quad x = term(s);
+        h[0] += x.x;
+        h[1] += x.y;
+        h[2] += x.z;
+      }
+#pragma unroll
+      for (int j = 0; j < 3; ++j) {
+        h[j] = fb_warp_sum(h[j]);
+        if (lane == k) g[j] = h[j];
+      }
     }
-    A.g[3 * t] = g0;
-    A.g[3 * t + 1] = g1;
-    A.g[3 * t + 2] = g2;
+    if (t < n1) {
+      double2* o = reinterpret_cast<double2*>(A.g + 4 * t);
+      o[0] = make_double2(g[0] / v0, g[1] / v0);
+      o[1] = make_double2(g[2] / v0, A.kappa * v0);
+    }
   }
 }
 
-__global__ void __launch_bounds__(kFbThreads) fbar_element(FbarArgs A) {
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < A.E; e += (int64_t)gridDim.x * blockDim.x) {
+constexpr int kFbElemThreads = 64;  // 52 KB of staged records: four blocks per SM, as the registers allow
+constexpr int kFbRecStride = kFbRec + 1;
+__global__ void __launch_bounds__(kFbElemThreads, 4) fbar_element(FbarArgs A) {
+  extern __shared__ __align__(16) double s_rec[];
+  const int64_t e0 = blockIdx.x * (int64_t)kFbElemThreads, e = e0 + threadIdx.x;
+  if (e < A.E) {
     const int4 cn = reinterpret_cast<const int4*>(A.conn)[e];
     double Xn[4][3], Un[4][3], g[4][3], F[3][3], detD;
     fb_nodes(A.X, cn, Xn);
@@ -254,7 +332,7 @@ __global__ void __launch_bounds__(kFbThreads) fbar_element(FbarArgs A) {
     }
     const double Ap = A.kappa + (2.0 / 9.0) * phib * I1b;
     const double Bp = (2.0 / 3.0) * phib * I1b - 2.0 * A.kappa * lnJb;
-    double* R = A.rec + (int64_t)kFbRec * e;
+    double* R = s_rec + kFbRecStride * threadIdx.x;
     const int gid[4] = {cn.x, cn.y, cn.z, cn.w};
     int slot = 0;
 #pragma unroll
@@ -280,10 +358,10 @@ __global__ void __launch_bounds__(kFbThreads) fbar_element(FbarArgs A) {
             v[k][m] = V * x;
           }
         if (a == b) {
-          double* d = R + 54 + 6 * a;
+          double* d = R + kFbDiag + 6 * a;
           d[0] = v[0][0]; d[1] = v[0][1]; d[2] = v[0][2]; d[3] = v[1][1]; d[4] = v[1][2]; d[5] = v[2][2];
         } else {
-          double* o = R + 9 * slot;
+          double* o = R + kFbPair * slot;
           const bool swap = gid[a] > gid[b];  // rows = the node of smaller global id
 #pragma unroll
           for (int k = 0; k < 3; ++k)
@@ -302,9 +380,12 @@ __global__ void __launch_bounds__(kFbThreads) fbar_element(FbarArgs A) {
         w[i] = r2 * (Sb[i][0] * g[b][0] + Sb[i][1] * g[b][1] + Sb[i][2] * g[b][2]) +
                (1.0 - r2) * (trS / 3.0) * g[b][i];
 #pragma unroll
-      for (int k = 0; k < 3; ++k) R[78 + 3 * b + k] = V * (F[k][0] * w[0] + F[k][1] * w[1] + F[k][2] * w[2]);
+      for (int k = 0; k < 3; ++k) R[kFbForce + 4 * b + k] = V * (F[k][0] * w[0] + F[k][1] * w[1] + F[k][2] * w[2]);
     }
   }
+  __syncthreads();
+  fb_copy_records<kFbRec, kFbRecStride, kFbRec>(A.rec + (int64_t)kFbRec * e0, s_rec,
+                                                (int)min((int64_t)kFbElemThreads, A.E - e0), [](int j) { return j; });
 }
 
 struct FbarGather {
@@ -317,85 +398,148 @@ struct FbarGather {
   int64_t n_pairs, n_nodes;
 };
 
+__device__ __forceinline__ int4 fb_info(const int32_t* p) { return make_int4(__ldg(p), __ldg(p + 1), __ldg(p + 2), __ldg(p + 3)); }
+
+// The one-ring blocks are added to the volumetric part, which fbar_vol has written (two
+// terms: the same bits in either order).  kBatch records are loaded together; each sum stays
+// in ascending element order.
+constexpr int kFbBatch = 2;
 __global__ void __launch_bounds__(kFbThreads) fbar_gather(FbarGather G, const double* __restrict__ rec,
                                                           double* __restrict__ k_out, double* __restrict__ f_out) {
-  const int64_t total = G.n_pairs + G.n_nodes;
-  for (int64_t it = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; it < total; it += (int64_t)gridDim.x * blockDim.x) {
-    if (it < G.n_pairs) {
-      if (!k_out) continue;
-      const int32_t* info = G.pair_info2 + 4 * it;
+  const int64_t pairs = (G.n_pairs + 31) / 32 * 32;  // whole warps per kind
+  for (int64_t it = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; it < pairs + G.n_nodes;
+       it += (int64_t)gridDim.x * blockDim.x) {
+    if (it < pairs) {
+      if (!k_out || it >= G.n_pairs) continue;
+      const int4 info = fb_info(G.pair_info2 + 4 * it);
+      const int32_t s1 = __ldg(G.pair_ptr + it + 1);
       double acc[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-      for (int32_t s = G.pair_ptr[it]; s < G.pair_ptr[it + 1]; ++s) {
-        const int32_t c = G.pair_src[s];
-        const double* o = rec + (int64_t)kFbRec * (c >> 6) + 9 * (c & 63);
+      for (int32_t s = __ldg(G.pair_ptr + it); s < s1; s += kFbBatch) {
+        double v[kFbBatch][9];
 #pragma unroll
-        for (int j = 0; j < 9; ++j) acc[j] += o[j];
+        for (int b = 0; b < kFbBatch; ++b)
+          if (s + b < s1) {
+            const int32_t c = __ldg(G.pair_src + s + b);
+            const double2* o = reinterpret_cast<const double2*>(rec + (int64_t)kFbRec * (c >> 6) + kFbPair * (c & 63));
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const double2 x = __ldg(o + j);
+              v[b][2 * j] = x.x;
+              v[b][2 * j + 1] = x.y;
+            }
+            v[b][8] = __ldg(reinterpret_cast<const double*>(o + 4));
+          }
+#pragma unroll
+        for (int b = 0; b < kFbBatch; ++b)
+          if (s + b < s1) {
+#pragma unroll
+            for (int j = 0; j < 9; ++j) acc[j] += v[b][j];
+          }
       }
 #pragma unroll
-      for (int k = 0; k < 3; ++k) store3(k_out + info[0] + (int64_t)info[1] * k, acc[3 * k], acc[3 * k + 1], acc[3 * k + 2]);
+      for (int k = 0; k < 3; ++k) add3(k_out + info.x + (int64_t)info.y * k, acc[3 * k], acc[3 * k + 1], acc[3 * k + 2]);
 #pragma unroll
-      for (int m = 0; m < 3; ++m) store3(k_out + info[2] + (int64_t)info[3] * m, acc[m], acc[3 + m], acc[6 + m]);
+      for (int m = 0; m < 3; ++m) add3(k_out + info.z + (int64_t)info.w * m, acc[m], acc[3 + m], acc[6 + m]);
     } else {
-      const int64_t n = it - G.n_pairs;
-      const int32_t* info = G.node_info2 + 4 * n;
+      const int64_t n = it - pairs;
+      const int4 info = fb_info(G.node_info2 + 4 * n);
+      const int32_t s1 = __ldg(G.node_ptr + n + 1);
       double d[6] = {0, 0, 0, 0, 0, 0}, f[3] = {0, 0, 0};
-      for (int32_t s = G.node_ptr[n]; s < G.node_ptr[n + 1]; ++s) {
-        const int32_t c = G.node_src[s];
-        const double* R = rec + (int64_t)kFbRec * (c >> 4);
-        const int a = c & 15;
+      for (int32_t s = __ldg(G.node_ptr + n); s < s1; s += kFbBatch) {
+        double v[kFbBatch][9];
 #pragma unroll
-        for (int j = 0; j < 6; ++j) d[j] += R[54 + 6 * a + j];
+        for (int b = 0; b < kFbBatch; ++b)
+          if (s + b < s1) {
+            const int32_t c = __ldg(G.node_src + s + b);
+            const double2* R = reinterpret_cast<const double2*>(rec + (int64_t)kFbRec * (c >> 4));
+            const int a = c & 15;
 #pragma unroll
-        for (int k = 0; k < 3; ++k) f[k] += R[78 + 3 * a + k];
+            for (int j = 0; j < 3; ++j) {
+              const double2 x = __ldg(R + kFbDiag / 2 + 3 * a + j);
+              v[b][2 * j] = x.x;
+              v[b][2 * j + 1] = x.y;
+            }
+            const double2 y = __ldg(R + kFbForce / 2 + 2 * a);
+            v[b][6] = y.x;
+            v[b][7] = y.y;
+            v[b][8] = __ldg(reinterpret_cast<const double*>(R + kFbForce / 2 + 2 * a + 1));
+          }
+#pragma unroll
+        for (int b = 0; b < kFbBatch; ++b)
+          if (s + b < s1) {
+#pragma unroll
+            for (int j = 0; j < 6; ++j) d[j] += v[b][j];
+#pragma unroll
+            for (int k = 0; k < 3; ++k) f[k] += v[b][6 + k];
+          }
       }
-      if (k_out && info[1] > 0) {
+      if (k_out && info.y > 0) {
         const double full[9] = {d[0], d[1], d[2], d[1], d[3], d[4], d[2], d[4], d[5]};
 #pragma unroll
         for (int k = 0; k < 3; ++k)
-          store3(k_out + info[0] + (int64_t)info[1] * k, full[3 * k], full[3 * k + 1], full[3 * k + 2]);
+          add3(k_out + info.x + (int64_t)info.y * k, full[3 * k], full[3 * k + 1], full[3 * k + 2]);
       }
-      if (f_out) store3(f_out + 3 * (int64_t)info[2], f[0], f[1], f[2]);
+      if (f_out) store3(f_out + 3 * (int64_t)info.z, f[0], f[1], f[2]);
     }
   }
 }
 
-// two-ring block (b, c): K += sum_a (kappa v0_a) (g_a[b] g_a[c]^T), a ascending.  One
-// thread per two-ring entry t (the block of node b and its t-th two-ring neighbour; b
-// found by a binary search of nbr2_ptr), so that the threads of a warp update adjacent
-// blocks of the same rows.
+// two-ring block (b, c): K = sum_a (kappa v0_a) (g_a[b] g_a[c]^T), a ascending.  One thread
+// per two-ring entry t (the block of node b and its t-th two-ring neighbour).  A warp's blocks
+// are exchanged through shared memory and leave row by row, 32 consecutive values per store.
 __global__ void __launch_bounds__(kFbThreads) fbar_vol(int64_t N, const int32_t* __restrict__ nbr2_ptr,
                                                        const int32_t* __restrict__ vol_ptr,
                                                        const int32_t* __restrict__ vol_src,
-                                                       const double* __restrict__ v0, const double* __restrict__ g,
-                                                       double kappa, double* __restrict__ k_out) {
-  const int64_t n2 = nbr2_ptr[N];
-  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n2; t += (int64_t)gridDim.x * blockDim.x) {
-    // the node b with nbr2_ptr[b] <= t < nbr2_ptr[b + 1]
-    int64_t lo = 0, hi = N;
-    while (hi - lo > 1) {
-      const int64_t mid = (lo + hi) / 2;
-      if (nbr2_ptr[mid] <= t)
-        lo = mid;
-      else
-        hi = mid;
-    }
-    const int64_t b = lo;
-    const int32_t t0 = nbr2_ptr[b], t1 = nbr2_ptr[b + 1];
-    const int64_t row = 9 * (int64_t)t0, stride = 3 * (int64_t)(t1 - t0);
-    double acc[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-    for (int32_t s = vol_ptr[t]; s < vol_ptr[t + 1]; ++s) {
+                                                       const double* __restrict__ g, double* __restrict__ k_out) {
+  __shared__ double s_all[kFbThreads / 32][32 * 9];
+  __shared__ int64_t s_pos[kFbThreads / 32][32];
+  __shared__ int32_t s_stride[kFbThreads / 32][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  double* s_k = s_all[w];
+  const int64_t n2 = __ldg(nbr2_ptr + N);
+  for (int64_t t0 = blockIdx.x * (int64_t)kFbThreads + 32 * w; t0 < n2; t0 += (int64_t)gridDim.x * kFbThreads) {
+    const int64_t t = t0 + lane;
+    const int32_t s0 = __ldg(vol_ptr + min(t, n2)), s1 = __ldg(vol_ptr + min(t + 1, n2));
+    const int64_t b = fb_node_of(nbr2_ptr, N, t0, lane);
+    const int32_t p0 = __ldg(nbr2_ptr + b), p1 = __ldg(nbr2_ptr + b + 1);
+    s_stride[w][lane] = 3 * (p1 - p0);
+    s_pos[w][lane] = 9 * (int64_t)p0 + 3 * (t - p0);
+    auto add = [&](double acc[9], int32_t s) {
       const int32_t* v = vol_src + 3 * (int64_t)s;
-      const double sc = kappa * v0[v[0]];
-      const double* gb = g + 3 * (int64_t)v[1];
-      const double* gc = g + 3 * (int64_t)v[2];
+      const Quad gb = ld_quad_nc(g + 4 * (int64_t)__ldg(v + 1)), gc = ld_quad_nc(g + 4 * (int64_t)__ldg(v + 2));
+      const double b3[3] = {gb.x, gb.y, gb.z}, c3[3] = {gc.x, gc.y, gc.z};
 #pragma unroll
       for (int k = 0; k < 3; ++k)
 #pragma unroll
-        for (int m = 0; m < 3; ++m) acc[3 * k + m] += sc * (gb[k] * gc[m]);
+        for (int m = 0; m < 3; ++m) acc[3 * k + m] += gb.w * (b3[k] * c3[m]);
+    };
+    double acc[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+    if (s1 - s0 <= kFbLong) {
+#pragma unroll 2
+      for (int32_t s = s0; s < s1; ++s) add(acc, s);
     }
-    const int64_t col = 3 * (t - t0);
 #pragma unroll
-    for (int k = 0; k < 3; ++k) add3(k_out + row + stride * k + col, acc[3 * k], acc[3 * k + 1], acc[3 * k + 2]);
+    for (int j = 0; j < 9; ++j) s_k[9 * lane + j] = acc[j];
+    for (unsigned m = __ballot_sync(0xffffffffu, s1 - s0 > kFbLong); m; m &= m - 1) {
+      const int e = __ffs(m) - 1;
+      const int32_t a0 = __shfl_sync(0xffffffffu, s0, e), a1 = __shfl_sync(0xffffffffu, s1, e);
+      double sum[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+      for (int32_t s = a0 + lane; s < a1; s += 32) add(sum, s);
+#pragma unroll
+      for (int j = 0; j < 9; ++j) {
+        const double x = fb_warp_sum(sum[j]);
+        if (lane == e) s_k[9 * e + j] = x;
+      }
+    }
+    __syncwarp();
+    const int n = (int)min((int64_t)32, n2 - t0);
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+      for (int c = lane; c < 3 * n; c += 32) {
+        const int i = c / 3, m = c - 3 * i;
+        __stcs(k_out + s_pos[w][i] + (int64_t)s_stride[w][i] * k + m, s_k[9 * i + 3 * k + m]);
+      }
+    __syncwarp();
   }
 }
 
@@ -512,7 +656,7 @@ extern "C" int psx_fbar_element(int64_t n, const double* X_elem, const double* u
 }
 
 extern "C" int64_t psx_fbar_work_doubles(int64_t E, int64_t N, int64_t n_nbr) {
-  return 3 * E + 12 * E + 2 * N + E + 3 * n_nbr + (int64_t)psx::kFbRec * E;
+  return 4 * E + 2 * N + 16 * E + 4 * n_nbr + (int64_t)psx::kFbRec * E + 3;  // + 3: 32-byte alignment of q, g and records
 }
 
 extern "C" int psx_fbar_assemble(const int32_t* conn, int64_t E, int64_t N, const double* X, const double* u,
@@ -535,26 +679,31 @@ extern "C" int psx_fbar_assemble(const int32_t* conn, int64_t E, int64_t N, cons
   A.conn = conn; A.X = X; A.U = u; A.mu = mu; A.kappa = kappa;
   A.inc_ptr = inc_ptr; A.inc_elem = inc_elem; A.nbr_ptr = nbr_ptr; A.nbr = nbr;
   A.blk_ptr = blk_ptr; A.blk_src = blk_src; A.jbar_in = jbar_in;
-  double* w = work;
+  double* w = reinterpret_cast<double*>((reinterpret_cast<uintptr_t>(work) + 31) / 32 * 32);
+  A.rec = w; w += (int64_t)kFbRec * E;
+  A.q = w; w += 16 * E;
+  A.g = w; w += 4 * n_nbr;
   A.V = w; w += E;
   A.J = w; w += E;
-  A.Jbar = jbar_out ? jbar_out : w; w += E;
-  A.q = w; w += 12 * E;
   A.v0 = w; w += N;
   A.Jn = w; w += N;
-  A.g = w; w += 3 * n_nbr;
-  A.rec = w;
+  A.Jbar = jbar_out ? jbar_out : w;
   A.st = static_cast<Status*>(status);
   A.E = E; A.N = N;
   fbar_pre<<<fb_grid(E), kFbThreads, 0, s>>>(A);
   fbar_nodes<<<fb_grid(N), kFbThreads, 0, s>>>(A);
   if (k_out) fbar_patch<<<fb_grid(n_nbr), kFbThreads, 0, s>>>(A);  // one thread per one-ring entry
-  fbar_element<<<fb_grid(E), kFbThreads, 0, s>>>(A);
-  if (k_out && cudaMemsetAsync(k_out, 0, sizeof(double) * nnz2, s) != cudaSuccess) return PSX_ERR_CUDA;
+  // before the element pass, so that the records are still in L2 when they are gathered; the
+  // two-ring CSR holds 9 values per entry
+  if (k_out)
+    fbar_vol<<<fb_grid(nnz2 / 9), kFbThreads, 0, s>>>(N, nbr2_ptr, vol_ptr, vol_src, A.g, k_out);
+  constexpr int kElemSmem = sizeof(double) * kFbElemThreads * kFbRecStride;
+  static unsigned long long s_smem_set = 0;
+  if (set_dynamic_smem_once(fbar_element, kElemSmem, &s_smem_set) != cudaSuccess) return PSX_ERR_CUDA;
+  if ((E + kFbElemThreads - 1) / kFbElemThreads > 0x7fffffff) return PSX_ERR_LIMIT;
+  fbar_element<<<(unsigned)((E + kFbElemThreads - 1) / kFbElemThreads), kFbElemThreads, kElemSmem, s>>>(A);
   FbarGather G{pair_info2, pair_ptr, pair_src, node_info2, node_ptr, node_src, n_pairs, N};
   fbar_gather<<<fb_grid(n_pairs + N), kFbThreads, 0, s>>>(G, A.rec, k_out, f_out);
-  // one thread per two-ring entry: the two-ring CSR holds 9 values per entry
-  if (k_out) fbar_vol<<<fb_grid(nnz2 / 9), kFbThreads, 0, s>>>(N, nbr2_ptr, vol_ptr, vol_src, A.v0, A.g, kappa, k_out);
   PSX_CUDA_CHECK_LAUNCH();
   return PSX_OK;
 }

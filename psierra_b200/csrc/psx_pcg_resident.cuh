@@ -164,14 +164,6 @@ struct ResArgs {
   int32_t maxiter, identity;
 };
 
-// Three doubles of a padded node of p: the first by a 16-byte load.  Plain (L1) loads: the
-// meeting before the product acquires the other blocks' writes, and a node's p is read by
-// its neighbours in this block as well.
-__device__ __forceinline__ void res_node(const double* p, double x[3]) {
-  asm volatile("ld.global.v2.f64 {%0, %1}, [%2];" : "=d"(x[0]), "=d"(x[1]) : "l"(p));
-  asm volatile("ld.global.f64 %0, [%1];" : "=d"(x[2]) : "l"(p + 2));
-}
-
 // Matrix values and columns, each read once per product: not kept in L1, which is p's.
 __device__ __forceinline__ float res_once(const float* p) {
   float v;
@@ -242,11 +234,12 @@ __global__ void __launch_bounds__(res_threads<CLUSTER>(), 1) pcg_resident(ResArg
             v[3 + m] = res_once(q + len + m);
             v[6 + m] = res_once(q + 2 * len + m);
           }
-          double x[3];
-          res_node(A.p + 4 * (int64_t)(c / 3), x);
+          // a plain (L1) load: the meeting before the product acquires the other blocks'
+          // writes, and a node's p is read by its neighbours in this block as well
+          const Quad x = ld_quad(A.p + 4 * (int64_t)(c / 3));
 #pragma unroll
           for (int m = 0; m < 3; ++m)
-            a[m] += (double)v[3 * m] * x[0] + (double)v[3 * m + 1] * x[1] + (double)v[3 * m + 2] * x[2];
+            a[m] += (double)v[3 * m] * x.x + (double)v[3 * m + 1] * x.y + (double)v[3 * m + 2] * x.z;
         }
 #pragma unroll
         for (int m = 0; m < 3; ++m) {
