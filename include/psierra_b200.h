@@ -168,6 +168,8 @@ typedef struct psx_plan {
      node sums) on records of the whole mesh, without queue or waits; psx_work_bytes counts
      those records.  The values are the queued kernels' bit for bit. */
   int32_t two_pass;
+  int32_t two_pass_k;       /* the same for the FP32 tangent sweeps of psx_tet4_assemble[_effective] */
+  int32_t reserved0;        /* 0 */
 } psx_plan_t;
 
 /* n_pairs = (sum deg - N) / 2 and the pair_src length E * npe (npe - 1) / 2 (host). */

@@ -134,6 +134,8 @@ class PlanStruct(ctypes.Structure):
         ("gtasks_k", ctypes.c_void_p),
         ("wait_spins", ctypes.c_int32),
         ("two_pass", ctypes.c_int32),
+        ("two_pass_k", ctypes.c_int32),
+        ("reserved0", ctypes.c_int32),
     ]
 
 

@@ -109,14 +109,14 @@ class GPUAssembler:
                   ring_slack: int | None = None, lag_f: int | None = None, split: bool | None = None) -> None:
         """Launch shape of the persistent kernel (see ``MeshPattern.set_queue``)."""
         p = self.pattern
-        old = (p.lag, p.lag_f, p.ring_slack, p.two_pass)
+        old = (p.lag, p.lag_f, p.ring_slack, p.two_pass, p.two_pass_k)
         p.set_queue(lag=lag, blocks_per_sm=blocks_per_sm, ring_slack=ring_slack, lag_f=lag_f, split=split)
-        if (p.lag, p.lag_f, p.ring_slack, p.two_pass) != old:
+        if (p.lag, p.lag_f, p.ring_slack, p.two_pass, p.two_pass_k) != old:
             self._work.clear()  # the records are sized by the lag, the slack and the passes
 
-    def set_two_pass(self) -> None:
+    def set_two_pass(self, f: bool = True, k: bool = True) -> None:
         """Back to the two-pass sweeps after ``set_queue`` (see ``MeshPattern.two_pass``)."""
-        self.pattern.set_two_pass()
+        self.pattern.set_two_pass(f, k)
         self._work.clear()
 
     def set_wait_limit(self, spins: int) -> None:

@@ -80,7 +80,7 @@ def tune(asm, u: torch.Tensor, precision: str | None = None, want_f: bool = True
         hit = tuple(hit) + (asm.pattern.split,) * (4 - len(hit))
         _apply(asm, want_k, *hit[:4])
         if len(hit) > 4 and hit[4]:
-            asm.set_two_pass()
+            asm.set_two_pass(f=not want_k, k=want_k)
         return {"lag": hit[0], "blocks_per_sm": hit[1], "ring_slack": hit[2], "split": hit[3], "ms": None,
                 "table": {}}
     f = asm.new_f() if want_f else None
@@ -97,10 +97,11 @@ def tune(asm, u: torch.Tensor, precision: str | None = None, want_f: bool = True
     best = min(table, key=table.get)
     entry = best
     _apply(asm, want_k, *best)
-    if asm.npe == 4 and not want_k and hasattr(asm, "set_two_pass"):
-        # the sweeps without a tangent also run without a queue: keep the faster way
-        asm.set_two_pass()
-        if _time(asm, u, prec, want_f, want_k, f, k, reps) < table[best]:
+    if asm.npe == 4 and hasattr(asm, "set_two_pass"):
+        # sweeps that also run in two passes, without a queue: keep the faster way
+        asm.set_two_pass(f=not want_k, k=want_k)
+        if (asm.pattern.two_pass_k and prec == "fp32-mixed" if want_k else asm.pattern.two_pass) and \
+                _time(asm, u, prec, want_f, want_k, f, k, reps) < table[best]:
             entry = best + (True,)
         else:
             _apply(asm, want_k, *best)

@@ -58,6 +58,10 @@ __device__ __forceinline__ double det3(const double a[3][3]) {
                a[0][2], dmm(a[1][0], a[2][1], a[1][1], a[2][0]));
 }
 
+// Constant divisors as products with the rounded reciprocal: an FP64 division is a dozen
+// instructions and a branch on the FP64 pipe, and these quotients carry half an ulp either way.
+constexpr double kThird = 1.0 / 3.0, kSixth = 1.0 / 6.0;
+
 // Inverse through the adjugate; returns the determinant.
 __device__ __forceinline__ double inv3(const double a[3][3], double r[3][3]) {
   const double c00 = dmm(a[1][1], a[2][2], a[1][2], a[2][1]);
@@ -70,7 +74,7 @@ __device__ __forceinline__ double inv3(const double a[3][3], double r[3][3]) {
   const double c21 = dmm(a[0][1], a[2][0], a[0][0], a[2][1]);
   const double c22 = dmm(a[0][0], a[1][1], a[0][1], a[1][0]);
   const double det = ddot3(a[0][0], c00, a[0][1], c10, a[0][2], c20);
-  const double id = 1.0 / det;
+  const double id = __drcp_rn(det);
   r[0][0] = dmul(c00, id); r[0][1] = dmul(c01, id); r[0][2] = dmul(c02, id);
   r[1][0] = dmul(c10, id); r[1][1] = dmul(c11, id); r[1][2] = dmul(c12, id);
   r[2][0] = dmul(c20, id); r[2][1] = dmul(c21, id); r[2][2] = dmul(c22, id);
@@ -124,7 +128,7 @@ __device__ __forceinline__ void neohookean_point(const double l[3][3], double mu
   s.I1 = dfma(2.0, trE, 3.0);
   // T = 2 phi dev E + beta I (symmetric)
   double T[3][3];
-  const double tw = dmul(2.0, s.phi), dia = dfma(-tw, trE / 3.0, s.beta);
+  const double tw = dmul(2.0, s.phi), dia = dfma(-tw, dmul(trE, kThird), s.beta);
 #pragma unroll
   for (int i = 0; i < 3; ++i)
 #pragma unroll
@@ -151,7 +155,7 @@ template <typename T>
 __device__ __forceinline__ TangentCoef<T> tangent_coef(const PointState& s, double kappa, double w) {
   TangentCoef<T> t;
   t.A = (T)dmul(w, dfma(dmul(2.0 / 9.0, s.phi), s.I1, kappa));
-  t.hb = (T)dmul(w, dsub(dmul(s.phi, s.I1) / 3.0, s.beta));
+  t.hb = (T)dmul(w, dsub(dmul(dmul(s.phi, s.I1), kThird), s.beta));
   t.c = (T)dmul(w, dmul(-2.0 / 3.0, s.phi));
   t.phi = (T)dmul(w, s.phi);
   return t;

@@ -774,7 +774,7 @@ inline int work_layout(const psx_plan_t* P, int precision, void* work, WorkLayou
   const int32_t lag = queue_k || P->lag_f <= 0 ? P->lag : P->lag_f;
   while (ring < W->span_g + lag + slack) ring <<= 1;
   // two-pass sweeps keep the records of the whole mesh
-  const bool whole = P->two_pass && P->npe == 4 && !queue_k;
+  const bool whole = P->npe == 4 && (queue_k ? P->two_pass_k && precision == PSX_FP32_MIXED : P->two_pass);
   W->ring_g = ring < all && !whole ? ring : all;
   W->ring_elems = (int64_t)W->ring_g * P->granule;
   const int sms = device_sm_count();

@@ -349,7 +349,17 @@ __device__ __forceinline__ void tile_meta_prefetch(const GatherArgs& g, int64_t 
 // planes (gather_args): pair values 0-3, 4-7 and 8, diagonal xx xy xz yy and yz zz, and
 // f x, y, z, each plane contiguous over the tile's pairs or nodes, so that every store
 // of the warp writes whole sectors.
-template <bool WANT_K, bool WANT_F>
+template <bool KEEP, typename V>
+__device__ __forceinline__ void st_record(V* q, V v) {
+  if constexpr (KEEP)
+    st_ring(q, v);
+  else
+    __stcg(q, v);
+}
+
+// KEEP: with the L2 evict_last policy of the ring; records of the whole mesh take plain L2
+// stores (3.07M elements: f 167 -> 165 us, K.v 221 -> 218).
+template <bool WANT_K, bool WANT_F, bool KEEP = true>
 __device__ __forceinline__ void tile_reduce(const GatherArgs& g, int64_t t, const unsigned char* __restrict__ lst,
                                             const float* __restrict__ kst, const double* __restrict__ fst,
                                             float* __restrict__ krec, double* __restrict__ frec) {
@@ -377,9 +387,9 @@ __device__ __forceinline__ void tile_reduce(const GatherArgs& g, int64_t t, cons
         s1.x += y.x; s1.y += y.y; s1.z += y.z; s1.w += y.w;
         s2 += b[8];
       }
-      st_ring(p0 + lp, s0);
-      st_ring(p1 + lp, s1);
-      st_ring(p2 + lp, s2);
+      st_record<KEEP>(p0 + lp, s0);
+      st_record<KEEP>(p1 + lp, s1);
+      st_record<KEEP>(p2 + lp, s2);
     }
   }
   const int nn = lst[1];
@@ -412,13 +422,13 @@ __device__ __forceinline__ void tile_reduce(const GatherArgs& g, int64_t t, cons
       }
     }
     if constexpr (WANT_K) {
-      st_ring(d0p + ln, d0);
-      st_ring(d1p + ln, d1);
+      st_record<KEEP>(d0p + ln, d0);
+      st_record<KEEP>(d1p + ln, d1);
     }
     if constexpr (WANT_F) {
-      st_ring(fb + ln, f0);
-      st_ring(fb + g.cap_n4 + ln, f1);
-      st_ring(fb + 2 * g.cap_n4 + ln, f2);
+      st_record<KEEP>(fb + ln, f0);
+      st_record<KEEP>(fb + g.cap_n4 + ln, f1);
+      st_record<KEEP>(fb + 2 * g.cap_n4 + ln, f2);
     }
   }
 }
@@ -561,44 +571,75 @@ tet4_split_kernel(Tet4Args A, GatherArgs g, QueueArgs Q, const int4* __restrict_
 }
 
 // ---- two-pass sweeps ------------------------------------------------------------------
-// The sweeps without a tangent (f, K.v, dynamic relaxation, adjoint) in two launches: one
-// warp per element tile writes its tile record, then one thread per node sums the records.
-// Same element code, records and association as the queue, so the same bits; but no
-// claims, waits or completion counts, warps that hold only what an element tile needs
-// (16-20 per SM), and gathers at full occupancy, 12 blocks of them behind each SM's loads
-// instead of a turn in the queue.  The records of the whole mesh are kept (22 bytes per
-// element, in L2 up to about 5M elements).  Measured, queue -> two passes, us:
-//   elements    f              K.v FP32        K.v FP64
-//     384,000    71 ->  28      69 ->  33       80 ->  35
-//   1,053,696   106 ->  64     120 ->  83      121 ->  84
-//   3,072,000   272 -> 174     297 -> 231      320 -> 231
-// What bounds them now is the latency of the FP64 element chain (47% issue; the FP64 pipe
-// alone would take 21 us at 1.05M elements).  Passing over the mesh in pieces, so that the
-// records stay in L2, only adds launches (1.05M elements, 16 pieces: f 104 us).
+// The sweeps without a tangent (f, K.v, dynamic relaxation, adjoint), and the FP32 tangents of
+// meshes whose records stay in L2, in two launches: one warp per element tile writes its tile
+// record, then one thread per pair / node sums the records.  Same element code, records and
+// association as the queue, so the same bits; but no claims, waits or completion counts, warps
+// that hold only what an element tile needs, and gathers at full occupancy instead of a turn
+// in the queue.  The records of the whole mesh are kept (22 bytes per element without a
+// tangent, in L2 up to about 5M elements; 141 with one, so larger meshes queue:
+// psierra_b200/pattern.py has the line).  Measured, queue -> two passes, us:
+//   elements    f              K.v FP32        K.v FP64      f + K FP32
+//     384,000    71 ->  25      69 ->  31       80 ->  33     119 ->  91
+//   1,053,696   106 ->  56     120 ->  68      121 ->  80     237 -> 244 (queued)
+//   3,072,000   272 -> 146     297 -> 181      320 -> 220     639 -> 672 (queued)
+// What bounds them now: without a tangent the latency of the FP64 element chain (the FP64
+// pipe alone would take 21 us at 1.05M elements); with one, half each, pass 1 at 12 warps per
+// SM (shared memory of the staged blocks) and the scattered record reads and 12-byte row
+// segments of pass 2.  Passing over the mesh in pieces only adds launches (f, 1.05M elements,
+// 16 pieces: 104 us).
+// Resident blocks per SM that pass 1's registers are held to: 7 (72 registers) for f and the
+// FP32 products (3.07M elements: f 165 us at 4, 153 at 6, 146 at 7, 154 at 8; K.v 219, 185,
+// 181 and 196), 4 for the FP64 product, which spills below 128 registers (K.v 221 us at 4, 294
+// at 5), 3 for the FP32 tangents (the staged blocks' shared memory), 2 for the adjoint.
 template <typename KT, int MODE>
-__global__ void __launch_bounds__(kThreads, min_blocks<KT, MODE>())
-tet4_tiles_kernel(Tet4Args A, GatherArgs g, int64_t n_elements, double* __restrict__ frec) {
+constexpr int tiles_blocks() {
+  return (MODE & kModeAdjoint) != 0                   ? 2
+         : (MODE & PSX_KV) != 0                       ? (sizeof(KT) == 8 ? 4 : 7)
+         : (MODE & PSX_WANT_K) != 0                   ? 3
+                                                      : 7;
+}
+
+template <typename KT, int MODE>
+__global__ void __launch_bounds__(kThreads, tiles_blocks<KT, MODE>())
+tet4_tiles_kernel(Tet4Args A, GatherArgs g, int64_t n_elements, float* __restrict__ krec, double* __restrict__ frec) {
   using S = Tet4Smem<KT, MODE>;
-  static_assert(S::kTiles && !S::kWantK, "tile records of a sweep without a tangent");
+  static_assert(S::kTiles, "tile records");
   const int lane = threadIdx.x & 31;
   extern __shared__ __align__(16) unsigned char s_stage[];
   unsigned char* my_stage = s_stage + (threadIdx.x >> 5) * S::kWarpBytes;
-  double* fst = reinterpret_cast<double*>(my_stage);
-  unsigned char* lst = my_stage + sizeof(double) * S::kFDoubles;
+  float* kst = reinterpret_cast<float*>(my_stage);
+  double* fst = reinterpret_cast<double*>(my_stage + sizeof(float) * S::kKFloats);
+  unsigned char* lst = my_stage + sizeof(float) * S::kKFloats + sizeof(double) * S::kFDoubles;
   const int64_t t = blockIdx.x * (int64_t)(kThreads / 32) + (threadIdx.x >> 5);
   const int64_t e0 = t * g.tile;
   if (e0 >= n_elements) return;
-  tile_meta_prefetch<false>(g, t, lst);
+  tile_meta_prefetch<S::kWantK>(g, t, lst);
   const int64_t e = e0 + lane;
   if (lane < g.tile && e < n_elements)
-    tet4_element<KT, MODE, false, false>(A, e, __ldg(reinterpret_cast<const int4*>(A.conn) + e), nullptr,
-                                         fst + kFStride * lane);
+    tet4_element<KT, MODE, false, false>(A, e, __ldg(reinterpret_cast<const int4*>(A.conn) + e),
+                                         reinterpret_cast<KT*>(kst + lane * kStageStride), fst + kFStride * lane);
   cp_async_wait_all();
   __syncwarp();
-  tile_reduce<false, true>(g, t, lst, nullptr, fst, nullptr, frec);
+  tile_reduce<S::kWantK, S::kWantF, false>(g, t, lst, kst, fst, krec, frec);
 }
 
+// Pass 2 of a tangent: one thread per pair, then per node.
 constexpr int kItemThreads = 128;
+template <int MODE>
+__global__ void __launch_bounds__(kItemThreads)
+tet4_items_kernel(GatherArgs g, int32_t n_pairs, int32_t n_nodes, const float* __restrict__ krec,
+                  const double* __restrict__ frec, float* __restrict__ k_out, double* __restrict__ f_out) {
+  constexpr bool kWantF = (MODE & PSX_WANT_F) != 0;
+  const int32_t pairs = (n_pairs + 31) / 32 * 32;  // whole warps per kind
+  const int32_t i = blockIdx.x * kItemThreads + threadIdx.x;
+  if (i < pairs) {
+    if (i < n_pairs) gather_pair<float, 4, true, kWantF, 2, true>(g, pair_head<true>(g, i), krec, k_out);
+  } else if (i - pairs < n_nodes) {
+    gather_node<float, 4, true, kWantF, false, true, 2, true>(g, node_head<true>(g, i - pairs), krec, frec, k_out, f_out);
+  }
+}
+
 template <int MODE>
 __global__ void __launch_bounds__(kItemThreads)
 tet4_nodes_kernel(GatherArgs g, int32_t n_nodes, const double* __restrict__ frec, double* __restrict__ f_out, DRArgs dr) {
@@ -609,19 +650,26 @@ tet4_nodes_kernel(GatherArgs g, int32_t n_nodes, const double* __restrict__ frec
 }
 
 template <typename KT, int MODE>
-int run_two_pass(const psx_plan_t* P, const Tet4Args& A, const WorkLayout& W, double* f_out, cudaStream_t stream,
-                 const DRArgs& dr) {
+int run_two_pass(const psx_plan_t* P, const Tet4Args& A, const WorkLayout& W, float* k_out, double* f_out,
+                 cudaStream_t stream, const DRArgs& dr) {
   using S = Tet4Smem<KT, MODE>;
   const GatherArgs g = gather_args(P, W.ring_elems);
-  if (!W.tiles || P->tile > 32 || g.meta_stride > kMetaBytes || P->n_nodes > 0x7fffffff) return PSX_ERR_ARG;
+  if (!W.tiles || P->tile > 32 || g.tile_k % 4 || g.meta_stride > kMetaBytes || P->n_pairs + P->n_nodes > 0x7fffff00)
+    return PSX_ERR_ARG;
   const size_t smem = (kThreads / 32) * S::kWarpBytes;
   static unsigned long long s_smem_set = 0;
   if (set_dynamic_smem_once(tet4_tiles_kernel<KT, MODE>, (int)smem, &s_smem_set) != cudaSuccess) return PSX_ERR_CUDA;
   const int64_t tiles = (P->n_elements + P->tile - 1) / P->tile, per_block = kThreads / 32;
   tet4_tiles_kernel<KT, MODE><<<(unsigned)((tiles + per_block - 1) / per_block), kThreads, smem, stream>>>(
-      A, g, P->n_elements, W.frec);
-  tet4_nodes_kernel<MODE><<<(unsigned)((P->n_nodes + kItemThreads - 1) / kItemThreads), kItemThreads, 0, stream>>>(
-      g, (int32_t)P->n_nodes, W.frec, f_out, dr);
+      A, g, P->n_elements, static_cast<float*>(W.krec), W.frec);
+  if constexpr (S::kWantK) {
+    const int64_t items = (P->n_pairs + 31) / 32 * 32 + P->n_nodes;
+    tet4_items_kernel<MODE><<<(unsigned)((items + kItemThreads - 1) / kItemThreads), kItemThreads, 0, stream>>>(
+        g, (int32_t)P->n_pairs, (int32_t)P->n_nodes, static_cast<const float*>(W.krec), W.frec, k_out, f_out);
+  } else {
+    tet4_nodes_kernel<MODE><<<(unsigned)((P->n_nodes + kItemThreads - 1) / kItemThreads), kItemThreads, 0, stream>>>(
+        g, (int32_t)P->n_nodes, W.frec, f_out, dr);
+  }
   PSX_CUDA_CHECK_LAUNCH();
   return PSX_OK;
 }
@@ -668,7 +716,7 @@ int run_tet4(const psx_plan_t* P, const Tet4Args& A, const WorkLayout& W, KT* k_
       (MODE & (PSX_WANT_K | PSX_LINEAR | PSX_MASS)) != 0 && (MODE & (PSX_KV | kModeAdjoint)) == 0;
   // every sweep without a tangent is faster in two passes (tet4_tiles_kernel), at all sizes
   if constexpr (!kWantK) {
-    if (P->two_pass) return run_two_pass<KT, MODE>(P, A, W, f_out, stream, dr);
+    if (P->two_pass) return run_two_pass<KT, MODE>(P, A, W, nullptr, f_out, stream, dr);
   }
   const GatherArgs g = gather_args(P, W.ring_elems);
   const QueueArgs Q = queue_args(P, W, kWantK);
@@ -724,6 +772,7 @@ int run_tet4_split(const psx_plan_t* P, const Tet4Args& A, const WorkLayout& W, 
 template <int MODE>
 int run_tet4_k32(const psx_plan_t* P, const Tet4Args& A, const WorkLayout& W, float* k_out, double* f_out,
                  cudaStream_t stream) {
+  if (P->two_pass_k && W.tiles) return run_two_pass<float, MODE>(P, A, W, k_out, f_out, stream, DRArgs{});
   if (P->gtasks_k && P->n_gtasks_k > 0 && W.tiles && split_usable<float, MODE>())
     return run_tet4_split<float, MODE>(P, A, W, k_out, f_out, stream);
   return run_tet4<float, MODE>(P, A, W, k_out, f_out, stream);

@@ -33,7 +33,7 @@ __device__ __forceinline__ void tet4_geometry(const double Xn[4][3], Tet4Geom& G
 #pragma unroll
     for (int j = 0; j < 3; ++j) D[i][j] = dsub(Xn[j + 1][i], Xn[0][i]);
   G.detD = inv3(D, Di);
-  G.V = G.detD / 6.0;
+  G.V = dmul(G.detD, kSixth);
 #pragma unroll
   for (int j = 0; j < 3; ++j) {
     G.g[1][j] = Di[0][j];
@@ -262,7 +262,7 @@ __device__ __forceinline__ void tet4_vjp(const Tet4Args& A, int64_t e, bool para
         FTL += ps.Finv[j][i] * Lw[i][j];
         double fd = 0.0;  // (F^-T dev E)[i][j]
 #pragma unroll
-        for (int k = 0; k < 3; ++k) fd += ps.Finv[k][i] * (E[k][j] - (k == j ? trE / 3.0 : 0.0));
+        for (int k = 0; k < 3; ++k) fd += ps.Finv[k][i] * (E[k][j] - (k == j ? trE * kThird : 0.0));
         FDL += fd * Lw[i][j];
       }
     if (A.dmu) A.dmu[e] = G.V * 2.0 * jm23 * FDL;

@@ -54,6 +54,7 @@ class MeshPattern:
         self._blocks: tuple | None = None
         self._plan_host: dict | None = None
         self.queued_f = False  # a lag of the f / K.v queue was chosen (set_queue)
+        self.queued_k = False  # a lag of the K queue or one of its kernels was chosen
         self.granule, self.tile, self.tile_items, self.lag, self.lag_f, self.ring_slack = self.QUEUE[npe]
         self.blocks_per_sm = 0
         self.wait_spins = 0  # polls of one bounded wait in the persistent kernels (0 = about a second)
@@ -209,7 +210,7 @@ class MeshPattern:
     def _apply_split(self, d: dict) -> None:
         st = d["plan"]
         on = self.split and d.get("n_gtasks_k", 0) > 0
-        st.two_pass = int(self.two_pass)
+        st.two_pass, st.two_pass_k = int(self.two_pass), int(self.two_pass_k)
         st.n_gtasks_k = d["n_gtasks_k"] if on else 0
         st.gtasks_k = d["gtasks_k"].data_ptr() if on else None
 
@@ -219,9 +220,24 @@ class MeshPattern:
         lag of their queue is chosen (``set_queue(lag_f=...)``) or its waits are limited."""
         return self.npe == 4 and not self.queued_f and self.wait_spins == 0
 
-    def set_two_pass(self) -> None:
-        """Back to the two-pass sweeps after ``set_queue``; a workspace must be re-queried."""
-        self.queued_f = False
+    # Elements up to which the FP32 tangent sweeps run in two passes too: their records (141
+    # bytes per element) then stay in L2 between the passes.  f + K on Kuhn cubes, us, two
+    # passes / queue: 82,944 elements 27 / 42, 196,608 47 / 85, 384,000 91 / 119, 663,552
+    # 159 / 209, 1,053,696 244 / 237, 3,072,000 672 / 639.
+    TWO_PASS_K_ELEMENTS = 3 << 18
+
+    @property
+    def two_pass_k(self) -> bool:
+        """The same for the Tet4 FP32 tangent sweeps of meshes up to ``TWO_PASS_K_ELEMENTS``:
+        until a lag of the K queue or one of its kernels (``set_queue(lag=..., split=...)``)
+        is chosen."""
+        return (self.npe == 4 and not self.queued_k and self.wait_spins == 0
+                and self.n_elements <= self.TWO_PASS_K_ELEMENTS)
+
+    def set_two_pass(self, f: bool = True, k: bool = True) -> None:
+        """Back to the two-pass sweeps (without and with a tangent) after ``set_queue``; a
+        workspace must be re-queried."""
+        self.queued_f, self.queued_k = self.queued_f and not f, self.queued_k and not k
         if self._dev is not None:
             self._apply_split(self._dev)
 
@@ -244,8 +260,9 @@ class MeshPattern:
         warp-specialised kernel (``split``; the mixed kernel otherwise).
 
         With ``lag_f``, the sweeps without a tangent run the queued kernel instead of two
-        passes (``set_two_pass`` goes back).  Rebuilds the task queues when a lag changes; a workspace sized for the old values
-        must be re-queried (``psx_work_bytes``) afterwards.
+        passes; with ``lag`` or ``split``, the FP32 tangent sweeps (``set_two_pass`` goes back).
+        Rebuilds the task queues when a lag changes; a workspace sized for the old values must
+        be re-queried (``psx_work_bytes``) afterwards.
         """
         rebuild = (lag is not None and int(lag) != self.lag) or (lag_f is not None and int(lag_f) != self.lag_f)
         for v in (lag, lag_f):
@@ -262,6 +279,8 @@ class MeshPattern:
             self.ring_slack = int(ring_slack)
         if split is not None:
             self.split = bool(split) and self.npe == 4
+        if lag is not None or split is not None:
+            self.queued_k = True
         if self._dev is not None:
             if rebuild:
                 self._build_tasks(self._dev)

@@ -1,7 +1,7 @@
 """Tet4 sweeps in two passes against the queued kernels (GPU).
 
-Same element code, tile records and association: f, K.v, dynamic relaxation and the adjoint
-must be equal bit for bit.  Meshes at the edges of the tiles: one element, a last tile of
+Same element code, tile records and association: f, K.v, dynamic relaxation, the adjoint and
+the FP32 tangents must be equal bit for bit.  Meshes at the edges of the tiles: one element, a last tile of
 one element, ragged boxes, shuffled numbering (wide spans, many nodes per tile), disjoint
 unions, a mesh of many granules.
 """
@@ -47,8 +47,9 @@ def _pair(mesh, precision):
     mu = np.random.default_rng(4).uniform(1e3, 5e3, mesh.n_elements)
     field = NeoHookeanField(mu, 20.0 * mu, mass_density=900.0)
     a, b = (GPUAssembler(mesh.nodes, mesh.elements, field, precision=precision) for _ in range(2))
-    b.set_queue(lag_f=b.pattern.lag_f)
-    assert a.dev["plan"].two_pass == 1 and b.dev["plan"].two_pass == 0
+    b.set_queue(lag_f=b.pattern.lag_f, split=True)
+    way = lambda s: (s.dev["plan"].two_pass, s.dev["plan"].two_pass_k)  # noqa: E731
+    assert way(a) == (1, 1) and way(b) == (0, 0)
     X = mesh.nodes
     ext = float(np.ptp(X, axis=0).max())
     u = 0.03 * (X[:, [1, 2, 0]] - X.mean(axis=0)) + 0.002 * ext * np.sin(6.0 * X / ext)
@@ -64,6 +65,12 @@ def test_two_pass_sweeps_equal_the_queued_kernels(name, precision):
     def sweeps(s):
         yield "f", s.assemble(u, want_k=False)[0]
         yield "K.v", s.kv(u, v)
+        yield from zip(("f of f+K", "K of f+K"), s.assemble(u))
+        yield "K", s.assemble(u, want_f=False)[1]
+        yield from zip(("f of effective", "effective"), s.assemble_effective(u, 0.9, 37.0, 0.02))
+        yield "effective without f", s.assemble_effective(u, 0.9, 37.0, 0.02, want_f=False)[1]
+        yield "mass", s.assemble(None, mass=True)[1]
+        yield "linear", s.assemble(None, linear=True)[1]
         yield from zip(("X", "mu", "kappa"), s.adjoint(u, v))
         x, vel, r = torch.zeros_like(v), torch.zeros_like(v), torch.empty_like(v)
         for _ in range(3):
@@ -84,6 +91,21 @@ def test_workspace_follows_the_way_the_sweeps_run():
     assert torch.equal(a.kv(u, v), y)
     a.set_wait_limit(1 << 22)
     assert a.dev["plan"].two_pass == 0 and torch.equal(a.kv(u, v), y)
+
+
+def test_larger_meshes_queue_their_fp32_tangent(monkeypatch):
+    from psierra_b200.pattern import MeshPattern
+
+    monkeypatch.setattr(MeshPattern, "TWO_PASS_K_ELEMENTS", 1000)
+    m = meshgen.box_tet4(1.0, 1.0, 1.0, 6, 6, 6)
+    mu = np.full(m.n_elements, 1e3)
+    a = GPUAssembler(m.nodes, m.elements, NeoHookeanField(mu, 20.0 * mu), precision="fp32-mixed")
+    assert a.dev["plan"].two_pass == 1 and a.dev["plan"].two_pass_k == 0
+    u = torch.zeros(3 * m.n_nodes, dtype=torch.float64, device=DEV)
+    k = a.assemble(u)[1]
+    monkeypatch.undo()
+    b = GPUAssembler(m.nodes, m.elements, NeoHookeanField(mu, 20.0 * mu), precision="fp32-mixed")
+    assert b.dev["plan"].two_pass_k == 1 and torch.equal(b.assemble(u)[1], k)
 
 
 def test_captured_in_a_graph():
