@@ -164,11 +164,12 @@ typedef struct psx_plan {
      returns at once).  0 = the default, 1 << 22 polls (about a second).  A small value
      lets a test make a wait run out without faulting the GPU. */
   int32_t wait_spins;
-  /* Non-zero: the Tet4 sweeps without a tangent run in two launches (element tiles, then
+  /* Non-zero: the sweeps without a tangent run in two launches (element tiles, then
      node sums) on records of the whole mesh, without queue or waits; psx_work_bytes counts
      those records.  The values are the queued kernels' bit for bit. */
   int32_t two_pass;
-  int32_t two_pass_k;       /* the same for the FP32 tangent sweeps of psx_tet4_assemble[_effective] */
+  int32_t two_pass_k;       /* the same for the FP32 tangent sweeps of psx_tet4_assemble[_effective]
+                               and all tangent sweeps of psx_tet10_assemble */
   int32_t reserved0;        /* 0 */
 } psx_plan_t;
 

@@ -102,8 +102,9 @@ class GPUAssembler:
 
     # ------------------------------------------------------------------ workspace
     def launches_per_call(self, precision: str | None = None) -> int:
-        """Kernel launches one assemble() call makes (one persistent kernel)."""
-        return 1
+        """Kernel launches of one assemble() of f and K: one persistent kernel, or two passes."""
+        two = self.pattern.two_pass_k and (self.npe == 10 or (precision or self.precision) == "fp32-mixed")
+        return 2 if two else 1
 
     def set_queue(self, lag: int | None = None, blocks_per_sm: int | None = None,
                   ring_slack: int | None = None, lag_f: int | None = None, split: bool | None = None) -> None:

@@ -62,20 +62,37 @@ struct GatherArgs {
 
 // 16-byte vector loads/stores of record blocks (L2-only loads: the ring is rewritten while
 // the kernel runs, so nothing may be served from a stale L1 line).
-template <typename KT, int N>
+//
+// CACHED: the records were written by an earlier launch (two-pass sweeps), so they may come
+// through L1: 32-byte loads of FP64 blocks (an L2-only 16-byte load fetches its 32-byte sector
+// each time, so each sector came twice), cached 16-byte loads of FP32 ones.
+template <bool CACHED, typename T>
+__device__ __forceinline__ T ld_rec(const T* p) {
+  if constexpr (CACHED)
+    return __ldg(p);
+  else
+    return __ldcg(p);
+}
+template <typename KT, int N, bool CACHED = false>
 __device__ __forceinline__ void load_block(const KT* __restrict__ p, KT v[N]) {
-  if constexpr (sizeof(KT) == 4) {
+  if constexpr (CACHED && sizeof(KT) == 8) {
+#pragma unroll
+    for (int i = 0; i < N / 4; ++i) {
+      const Quad t = ld_quad_nc(p + 4 * i);
+      v[4 * i] = t.x; v[4 * i + 1] = t.y; v[4 * i + 2] = t.z; v[4 * i + 3] = t.w;
+    }
+  } else if constexpr (sizeof(KT) == 4) {
     const float4* q = reinterpret_cast<const float4*>(p);
 #pragma unroll
     for (int i = 0; i < N / 4; ++i) {
-      const float4 t = __ldcg(q + i);
+      const float4 t = ld_rec<CACHED>(q + i);
       v[4 * i] = t.x; v[4 * i + 1] = t.y; v[4 * i + 2] = t.z; v[4 * i + 3] = t.w;
     }
   } else {
     const double2* q = reinterpret_cast<const double2*>(p);
 #pragma unroll
     for (int i = 0; i < N / 2; ++i) {
-      const double2 t = __ldcg(q + i);
+      const double2 t = ld_rec<CACHED>(q + i);
       v[2 * i] = t.x; v[2 * i + 1] = t.y;
     }
   }
@@ -170,7 +187,8 @@ __device__ __forceinline__ ItemHead node_head(const GatherArgs& g, int32_t n) {
 
 // Pair item: off-diagonal block and its transpose.  Contributions are summed in list
 // (ascending element) order; their loads are issued kBatch at a time.
-template <typename KT, int NPE, bool TILES = false, bool WANT_F = false, int BATCH = 0, bool VSTORE = false>
+template <typename KT, int NPE, bool TILES = false, bool WANT_F = false, int BATCH = 0, bool VSTORE = false,
+          bool CACHED = false>
 __device__ __forceinline__ void gather_pair(const GatherArgs& g, const ItemHead& h, const KT* __restrict__ krec,
                                             KT* __restrict__ k_out) {
   using L = RecLayout<NPE>;
@@ -193,17 +211,17 @@ __device__ __forceinline__ void gather_pair(const GatherArgs& g, const ItemHead&
           // pair planes of the tile record (K is FP32 wherever tile records hold K)
           const float* base = reinterpret_cast<const float*>(krec) + ((int64_t)(src[b] >> 8) & g.ring_tile_mask) * g.tile_k;
           const int lp = src[b] & 255;
-          const float4 x = __ldcg(reinterpret_cast<const float4*>(base) + lp);
-          const float4 y = __ldcg(reinterpret_cast<const float4*>(base + 4 * g.cap_p4) + lp);
+          const float4 x = ld_rec<CACHED>(reinterpret_cast<const float4*>(base) + lp);
+          const float4 y = ld_rec<CACHED>(reinterpret_cast<const float4*>(base + 4 * g.cap_p4) + lp);
           v[b][0] = x.x; v[b][1] = x.y; v[b][2] = x.z; v[b][3] = x.w;
           v[b][4] = y.x; v[b][5] = y.y; v[b][6] = y.z; v[b][7] = y.w;
-          v[b][8] = __ldcg(base + 8 * g.cap_p4 + lp);
+          v[b][8] = ld_rec<CACHED>(base + 8 * g.cap_p4 + lp);
         } else if constexpr (NPE == 4) {
           constexpr int W = 16 / (int)sizeof(KT);
           load_planes<KT, 12>(krec + ((int64_t)(src[b] >> 6) & g.ring_mask) * W, L::pair_off(src[b] & 63), v[b],
                               g.ring_mask + 1);
         } else {
-          load_block<KT, 12>(krec + ((int64_t)(src[b] >> 6) & g.ring_mask) * L::kK + L::pair_off(src[b] & 63), v[b]);
+          load_block<KT, 12, CACHED>(krec + ((int64_t)(src[b] >> 6) & g.ring_mask) * L::kK + L::pair_off(src[b] & 63), v[b]);
         }
       }
 #pragma unroll
@@ -241,7 +259,7 @@ struct DRArgs {
 
 // Node item: diagonal block and/or f (or, with DR, the fused pseudo-step on f = K x).
 template <typename KT, int NPE, bool WANT_K, bool WANT_F, bool DR = false, bool TILES = false, int BATCH = 0,
-          bool VSTORE = false>
+          bool VSTORE = false, bool CACHED = false>
 __device__ __forceinline__ void gather_node(const GatherArgs& g, const ItemHead& h, const KT* __restrict__ krec,
                                             const double* __restrict__ frec, KT* __restrict__ k_out,
                                             double* __restrict__ f_out, const DRArgs* dr = nullptr) {
@@ -269,16 +287,16 @@ __device__ __forceinline__ void gather_node(const GatherArgs& g, const ItemHead&
           const int ln = src[b] & 127;
           if constexpr (WANT_K) {
             const float* base = reinterpret_cast<const float*>(krec) + slot * g.tile_k + 9 * g.cap_p4;
-            const float4 x = __ldcg(reinterpret_cast<const float4*>(base) + ln);
-            const float2 y = __ldcg(reinterpret_cast<const float2*>(base + 4 * g.cap_n4) + ln);
+            const float4 x = ld_rec<CACHED>(reinterpret_cast<const float4*>(base) + ln);
+            const float2 y = ld_rec<CACHED>(reinterpret_cast<const float2*>(base + 4 * g.cap_n4) + ln);
             v[b][0] = x.x; v[b][1] = x.y; v[b][2] = x.z; v[b][3] = x.w;
             v[b][4] = y.x; v[b][5] = y.y;
           }
           if constexpr (WANT_F) {
             const double* fb = frec + slot * 3 * g.cap_n4 + ln;
-            fv[b][0] = __ldcg(fb);
-            fv[b][1] = __ldcg(fb + g.cap_n4);
-            fv[b][2] = __ldcg(fb + 2 * g.cap_n4);
+            fv[b][0] = ld_rec<CACHED>(fb);
+            fv[b][1] = ld_rec<CACHED>(fb + g.cap_n4);
+            fv[b][2] = ld_rec<CACHED>(fb + 2 * g.cap_n4);
           }
         } else if constexpr (NPE == 4) {
           // planar Tet4 element records (store_planes); f: value j of the 12 at granule j/2
@@ -291,7 +309,7 @@ __device__ __forceinline__ void gather_node(const GatherArgs& g, const ItemHead&
 #pragma unroll
             for (int j = 0; j < 3; ++j) {
               const int vj = 3 * a + j;
-              fv[b][j] = __ldcg(frec + slot * 2 + (int64_t)(vj >> 1) * plane * 2 + (vj & 1));
+              fv[b][j] = ld_rec<CACHED>(frec + slot * 2 + (int64_t)(vj >> 1) * plane * 2 + (vj & 1));
             }
           }
         } else {
@@ -299,11 +317,11 @@ __device__ __forceinline__ void gather_node(const GatherArgs& g, const ItemHead&
           const int a = src[b] & 15;
           const KT* kp = krec + slot * L::kK + L::diag_off(a);
           const double* fp = frec + slot * L::kF + 3 * a;
-          if constexpr (WANT_K) load_block<KT, 8>(kp, v[b]);
+          if constexpr (WANT_K) load_block<KT, 8, CACHED>(kp, v[b]);
           if constexpr (WANT_F) {
-            fv[b][0] = __ldcg(fp);
-            fv[b][1] = __ldcg(fp + 1);
-            fv[b][2] = __ldcg(fp + 2);
+            fv[b][0] = ld_rec<CACHED>(fp);
+            fv[b][1] = ld_rec<CACHED>(fp + 1);
+            fv[b][2] = ld_rec<CACHED>(fp + 2);
           }
         }
       }
@@ -774,7 +792,7 @@ inline int work_layout(const psx_plan_t* P, int precision, void* work, WorkLayou
   const int32_t lag = queue_k || P->lag_f <= 0 ? P->lag : P->lag_f;
   while (ring < W->span_g + lag + slack) ring <<= 1;
   // two-pass sweeps keep the records of the whole mesh
-  const bool whole = P->npe == 4 && (queue_k ? P->two_pass_k && precision == PSX_FP32_MIXED : P->two_pass);
+  const bool whole = queue_k ? P->two_pass_k && (P->npe == 10 || precision == PSX_FP32_MIXED) : P->two_pass;
   W->ring_g = ring < all && !whole ? ring : all;
   W->ring_elems = (int64_t)W->ring_g * P->granule;
   const int sms = device_sm_count();
@@ -796,8 +814,9 @@ inline int work_layout(const psx_plan_t* P, int precision, void* work, WorkLayou
     kbytes = queue_k ? up(ring_tiles * (9 * cp4 + 6 * cn4) * kt) : 0;
     fbytes = up(ring_tiles * 3 * cn4 * 8);
   } else {
-    kbytes = queue_k ? up(W->ring_elems * kK * kt) : 0;
-    fbytes = up(W->ring_elems * kF * 8);
+    const int64_t ring_elems = whole ? P->n_elements : W->ring_elems;
+    kbytes = queue_k ? up(ring_elems * kK * kt) : 0;
+    fbytes = up(ring_elems * kF * 8);
   }
   W->total_bytes = (int64_t)W->counter_bytes + kbytes + fbytes;
   W->counters = nullptr;

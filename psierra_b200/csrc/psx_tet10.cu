@@ -87,14 +87,68 @@ struct Tet10Args {
   Status* st;
 };
 
-// Shared-memory scratch of one warp: per (element, qp, node) p, q, H and per (element,
-// qp) the weighted tangent coefficients.
+// Shared-memory scratch of one warp: per (element, qp, node) a 48-byte record, per (element,
+// qp) the weighted tangent coefficients.  FP32: p, q, H as three 16-byte vectors.  FP64: p and
+// q as three pairs; H_a.H_b is formed as p_a.q_b (p = F^-T H, q = F H), which left the error of
+// the blocks against extended precision where it was (3.5e-14 of their norm at strains of
+// 0.2).  The block phase was bound by its 22 scalar loads per block and point (84% of the
+// kernel's shared-memory cycles, FP64); three vector loads per node take a third of them, and
+// 48 bytes keep consecutive nodes on distinct banks.  f + K, 162,000 elements, one launch:
+// 1035 -> 863 us FP64, 652 -> 639 us FP32; with H kept beside them 5 vectors: 797 us against
+// 736 (two passes).
 template <typename KT>
-struct Tet10Smem {
-  KT p[kTile10][4][10][3];
-  KT q[kTile10][4][10][3];
-  KT h[kTile10][4][10][3];
-  KT c[kTile10][4][4];  // A, hb, c, phi (times w det J)
+struct Tet10Smem;
+template <>
+struct Tet10Smem<float> {
+  float4 v[kTile10][4][10][3];
+  float4 c[kTile10][4];  // A, hb, c, phi (times w det J)
+  __device__ __forceinline__ void put(int e, int q, int a, const float p[3], const float qv[3], const float h[3]) {
+    v[e][q][a][0] = make_float4(p[0], p[1], p[2], 0.f);
+    v[e][q][a][1] = make_float4(qv[0], qv[1], qv[2], 0.f);
+    v[e][q][a][2] = make_float4(h[0], h[1], h[2], 0.f);
+  }
+  __device__ __forceinline__ void node(int e, int q, int a, float p[3], float qv[3], float h[3]) const {
+    const float4 x = v[e][q][a][0], y = v[e][q][a][1], z = v[e][q][a][2];
+    p[0] = x.x; p[1] = x.y; p[2] = x.z;
+    qv[0] = y.x; qv[1] = y.y; qv[2] = y.z;
+    h[0] = z.x; h[1] = z.y; h[2] = z.z;
+  }
+  __device__ __forceinline__ void put_coef(int e, int q, const TangentCoef<float>& t) {
+    c[e][q] = make_float4(t.A, t.hb, t.c, t.phi);
+  }
+  __device__ __forceinline__ TangentCoef<float> coef(int e, int q) const {
+    const float4 x = c[e][q];
+    return TangentCoef<float>{x.x, x.y, x.z, x.w};
+  }
+  static __device__ __forceinline__ float gram(const float[3], const float[3], const float ha[3], const float hb[3]) {
+    return ha[0] * hb[0] + ha[1] * hb[1] + ha[2] * hb[2];
+  }
+};
+template <>
+struct Tet10Smem<double> {
+  double2 v[kTile10][4][10][3];
+  double2 c[kTile10][4][2];
+  __device__ __forceinline__ void put(int e, int q, int a, const double p[3], const double qv[3], const double[3]) {
+    v[e][q][a][0] = make_double2(p[0], p[1]);
+    v[e][q][a][1] = make_double2(p[2], qv[0]);
+    v[e][q][a][2] = make_double2(qv[1], qv[2]);
+  }
+  __device__ __forceinline__ void node(int e, int q, int a, double p[3], double qv[3], double[3]) const {
+    const double2 x = v[e][q][a][0], y = v[e][q][a][1], z = v[e][q][a][2];
+    p[0] = x.x; p[1] = x.y; p[2] = y.x;
+    qv[0] = y.y; qv[1] = z.x; qv[2] = z.y;
+  }
+  __device__ __forceinline__ void put_coef(int e, int q, const TangentCoef<double>& t) {
+    c[e][q][0] = make_double2(t.A, t.hb);
+    c[e][q][1] = make_double2(t.c, t.phi);
+  }
+  __device__ __forceinline__ TangentCoef<double> coef(int e, int q) const {
+    const double2 x = c[e][q][0], y = c[e][q][1];
+    return TangentCoef<double>{x.x, x.y, y.x, y.y};
+  }
+  static __device__ __forceinline__ double gram(const double pa[3], const double qb[3], const double[3], const double[3]) {
+    return pa[0] * qb[0] + pa[1] * qb[1] + pa[2] * qb[2];
+  }
 };
 
 template <typename KT, int MODE>
@@ -245,24 +299,21 @@ __device__ __forceinline__ void tet10_tile(const Tet10Args& A, const int4& task,
     }
     if constexpr (kWantK) {
       const KT Hk[3] = {(KT)H[0], (KT)H[1], (KT)H[2]};
+      if constexpr (kLinear) {
+        sm.put(le, q, a, Hk, Hk, Hk);
+      } else {
+        KT pk[3], qk[3];
 #pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        sm.h[le][q][a][k] = Hk[k];
-        if constexpr (kLinear) {
-          sm.p[le][q][a][k] = Hk[k];
-          sm.q[le][q][a][k] = Hk[k];
-        } else {
-          sm.p[le][q][a][k] = Fi[0][k] * Hk[0] + Fi[1][k] * Hk[1] + Fi[2][k] * Hk[2];
-          sm.q[le][q][a][k] = Fm[k][0] * Hk[0] + Fm[k][1] * Hk[1] + Fm[k][2] * Hk[2];
+        for (int k = 0; k < 3; ++k) {
+          pk[k] = Fi[0][k] * Hk[0] + Fi[1][k] * Hk[1] + Fi[2][k] * Hk[2];
+          qk[k] = Fm[k][0] * Hk[0] + Fm[k][1] * Hk[1] + Fm[k][2] * Hk[2];
         }
+        sm.put(le, q, a, pk, qk, Hk);
       }
     }
   }
   if constexpr (kWantK) {
-    sm.c[le][q][0] = tc.A;
-    sm.c[le][q][1] = tc.hb;
-    sm.c[le][q][2] = tc.c;
-    sm.c[le][q][3] = tc.phi;
+    sm.put_coef(le, q, tc);
     __syncwarp();
     // ---- phase 2: blocks of the tile, summed over the 4 quadrature points
     const int n = (int)(task.w - task.z);
@@ -274,18 +325,17 @@ __device__ __forceinline__ void tet10_tile(const Tet10Args& A, const int4& task,
       for (int j = 0; j < 9; ++j) acc[j] = (KT)0;
 #pragma unroll
       for (int qq = 0; qq < 4; ++qq) {
-        const KT cA = sm.c[me][qq][0], chb = sm.c[me][qq][1], cc = sm.c[me][qq][2], cphi = sm.c[me][qq][3];
-        KT pa[3], pb[3], ha[3], ya[3], wb[3], s = 0;
+        const TangentCoef<KT> co = sm.coef(me, qq);
+        KT pa[3], qa[3], xa[3], pb[3], qb[3], xb[3], ha[3], ya[3], wb[3];
+        sm.node(me, qq, a, pa, qa, xa);
+        sm.node(me, qq, b, pb, qb, xb);
+        const KT s = co.phi * Tet10Smem<KT>::gram(pa, qb, xa, xb);
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
-          pa[k] = sm.p[me][qq][a][k];
-          pb[k] = sm.p[me][qq][b][k];
-          ha[k] = chb * pa[k];
-          ya[k] = cc * sm.q[me][qq][a][k];
-          wb[k] = cA * pb[k] + cc * sm.q[me][qq][b][k];
-          s += sm.h[me][qq][a][k] * sm.h[me][qq][b][k];
+          ha[k] = co.hb * pa[k];
+          ya[k] = co.c * qa[k];
+          wb[k] = co.A * pb[k] + co.c * qb[k];
         }
-        s *= cphi;
 #pragma unroll
         for (int k = 0; k < 3; ++k)
 #pragma unroll
@@ -314,6 +364,48 @@ tet10_persistent_kernel(Tet10Args A, GatherArgs g, QueueArgs Q, KT* __restrict__
   Tet10Smem<KT>& sm = reinterpret_cast<Tet10Smem<KT>*>(s_raw)[threadIdx.x >> 5];
   auto element_tile = [&](const int4& task) { tet10_tile<KT, MODE>(A, task, g.ring_mask, krec, frec, sm); };
   drain_queue<KT, 10, kWantK, kWantF, false, false>(g, Q, A.st, krec, frec, k_out, f_out, DRArgs{}, element_tile);
+}
+
+// Two passes, as psx_tet4.cu: element tiles (8 elements per one-warp block), then one thread
+// per pair / node.  The queue kept every SM at 8 warps (252 registers) for both phases and
+// its gathers, latency bound, waited on element tiles; split, a tile takes 168 registers and
+// no task (12 warps per SM), and the gathers run at their own occupancy with cached 32-byte
+// loads.  Kuhn cubes, us, one launch before / two passes: f + K FP64 384 elements 35 / 23,
+// 10,368 79 / 56, 162,000 1035 / 685, 750,000 4041 / 3280; FP32 162,000 652 / 493; f 384
+// elements 16 / 11, 162,000 200 / 76.  Tiles: 8 warps per SM 730 us (FP64 f + K, batches of
+// 2), 9 and more 708.  Pass 1 is bound by shared memory and FP64 latency, pass 2 by DRAM
+// (1.66 GB of records and values at 67% of the measured copy rate).
+template <typename KT, int MODE>
+constexpr int tiles10_blocks() {
+  return (MODE & PSX_MASS) != 0 ? 16 : sizeof(KT) == 8 && (MODE & (PSX_WANT_K | PSX_LINEAR)) != 0 ? 9 : 11;
+}
+template <typename KT, int MODE>
+__global__ void __launch_bounds__(32, (tiles10_blocks<KT, MODE>()))
+tet10_tiles_kernel(Tet10Args A, int64_t ring_mask, int64_t n_elements, KT* __restrict__ krec, double* __restrict__ frec) {
+  extern __shared__ __align__(16) unsigned char s_raw[];
+  const int64_t e0 = kTile10 * (int64_t)blockIdx.x;
+  tet10_tile<KT, MODE>(A, make_int4(0, 0, (int)e0, (int)min(e0 + kTile10, n_elements)), ring_mask, krec, frec,
+                       *reinterpret_cast<Tet10Smem<KT>*>(s_raw));
+}
+
+// Records in flight per thread: 3 (FP64 / FP32 f + K, 162,000 elements: 685 / 493 us; 1: 715 /
+// 510, 2: 697 / 504, 4: 686 / 493).
+constexpr int kItemThreads10 = 128, kItemBatch10 = 3;
+template <typename KT, int MODE>
+__global__ void __launch_bounds__(kItemThreads10)
+tet10_items_kernel(GatherArgs g, int32_t n_pairs, int32_t n_nodes, const KT* __restrict__ krec,
+                   const double* __restrict__ frec, KT* __restrict__ k_out, double* __restrict__ f_out) {
+  constexpr bool kWantF = (MODE & PSX_WANT_F) != 0;
+  constexpr bool kWantK = (MODE & (PSX_WANT_K | PSX_LINEAR | PSX_MASS)) != 0;
+  const int32_t pairs = kWantK ? (n_pairs + 31) / 32 * 32 : 0;  // whole warps per kind
+  const int32_t i = blockIdx.x * kItemThreads10 + threadIdx.x;
+  if (i < pairs) {
+    if constexpr (kWantK)
+      if (i < n_pairs) gather_pair<KT, 10, false, kWantF, kItemBatch10, true, true>(g, pair_head<false>(g, i), krec, k_out);
+  } else if (i - pairs < n_nodes) {
+    gather_node<KT, 10, kWantK, kWantF, false, false, kItemBatch10, true, true>(g, node_head<false>(g, i - pairs), krec,
+                                                                                frec, k_out, f_out);
+  }
 }
 
 // det J and det F at the 4 quadrature points of one element (error messages).
@@ -352,6 +444,17 @@ int run_tet10(const psx_plan_t* P, const Tet10Args& A, const WorkLayout& W, KT* 
               cudaStream_t stream) {
   constexpr bool kWantK = (MODE & (PSX_WANT_K | PSX_LINEAR | PSX_MASS)) != 0;
   const GatherArgs g = gather_args(P, W.ring_elems);
+  if (kWantK ? P->two_pass_k : P->two_pass) {
+    // f and the mass matrix stage nothing
+    const size_t smem = (MODE & (PSX_WANT_K | PSX_LINEAR)) != 0 ? sizeof(Tet10Smem<KT>) : 0;
+    tet10_tiles_kernel<KT, MODE><<<(unsigned)((P->n_elements + kTile10 - 1) / kTile10), 32, smem, stream>>>(
+        A, g.ring_mask, P->n_elements, static_cast<KT*>(W.krec), W.frec);
+    const int64_t items = (kWantK ? (P->n_pairs + 31) / 32 * 32 : 0) + P->n_nodes;
+    tet10_items_kernel<KT, MODE><<<(unsigned)((items + kItemThreads10 - 1) / kItemThreads10), kItemThreads10, 0, stream>>>(
+        g, (int32_t)P->n_pairs, (int32_t)P->n_nodes, static_cast<const KT*>(W.krec), W.frec, k_out, f_out);
+    PSX_CUDA_CHECK_LAUNCH();
+    return PSX_OK;
+  }
   const QueueArgs Q = queue_args(P, W, kWantK);
   if (cudaMemsetAsync(W.counters, 0, W.counter_bytes, stream) != cudaSuccess) return PSX_ERR_CUDA;
   const size_t smem = sizeof(Tet10Smem<KT>) * (kThreads10 / 32);

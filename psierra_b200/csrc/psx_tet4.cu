@@ -634,9 +634,9 @@ tet4_items_kernel(GatherArgs g, int32_t n_pairs, int32_t n_nodes, const float* _
   const int32_t pairs = (n_pairs + 31) / 32 * 32;  // whole warps per kind
   const int32_t i = blockIdx.x * kItemThreads + threadIdx.x;
   if (i < pairs) {
-    if (i < n_pairs) gather_pair<float, 4, true, kWantF, 2, true>(g, pair_head<true>(g, i), krec, k_out);
+    if (i < n_pairs) gather_pair<float, 4, true, kWantF, 2, true, true>(g, pair_head<true>(g, i), krec, k_out);
   } else if (i - pairs < n_nodes) {
-    gather_node<float, 4, true, kWantF, false, true, 2, true>(g, node_head<true>(g, i - pairs), krec, frec, k_out, f_out);
+    gather_node<float, 4, true, kWantF, false, true, 2, true, true>(g, node_head<true>(g, i - pairs), krec, frec, k_out, f_out);
   }
 }
 
@@ -645,8 +645,8 @@ __global__ void __launch_bounds__(kItemThreads)
 tet4_nodes_kernel(GatherArgs g, int32_t n_nodes, const double* __restrict__ frec, double* __restrict__ f_out, DRArgs dr) {
   const int32_t n = blockIdx.x * kItemThreads + threadIdx.x;
   if (n < n_nodes)
-    gather_node<double, 4, false, true, (MODE & kModeDR) != 0, true>(g, node_head<true>(g, n), nullptr, frec, nullptr,
-                                                                     f_out, &dr);
+    gather_node<double, 4, false, true, (MODE & kModeDR) != 0, true, 0, false, true>(g, node_head<true>(g, n), nullptr,
+                                                                                     frec, nullptr, f_out, &dr);
 }
 
 template <typename KT, int MODE>

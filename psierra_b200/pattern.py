@@ -216,23 +216,24 @@ class MeshPattern:
 
     @property
     def two_pass(self) -> bool:
-        """Whether the Tet4 sweeps without a tangent run in two passes: by default, until a
-        lag of their queue is chosen (``set_queue(lag_f=...)``) or its waits are limited."""
-        return self.npe == 4 and not self.queued_f and self.wait_spins == 0
+        """Whether the sweeps without a tangent run in two passes: by default, until a lag of
+        their queue is chosen (``set_queue(lag_f=...)``) or its waits are limited."""
+        return not self.queued_f and self.wait_spins == 0
 
-    # Elements up to which the FP32 tangent sweeps run in two passes too: their records (141
-    # bytes per element) then stay in L2 between the passes.  f + K on Kuhn cubes, us, two
+    # Elements up to which tangent sweeps run in two passes too.  Tet4, FP32: their records (141
+    # bytes per element) then stay in L2 between the passes; f + K on Kuhn cubes, us, two
     # passes / queue: 82,944 elements 27 / 42, 196,608 47 / 85, 384,000 91 / 119, 663,552
-    # 159 / 209, 1,053,696 244 / 237, 3,072,000 672 / 639.
+    # 159 / 209, 1,053,696 234 / 235, 3,072,000 652 / 630.  Tet10: two passes stay ahead (750,000
+    # elements, FP64, 3280 / 4000 us), but their records (5.2 KB per element) grow with the
+    # mesh, here to 4.1 GB; the queue's ring does not.
     TWO_PASS_K_ELEMENTS = 3 << 18
 
     @property
     def two_pass_k(self) -> bool:
-        """The same for the Tet4 FP32 tangent sweeps of meshes up to ``TWO_PASS_K_ELEMENTS``:
-        until a lag of the K queue or one of its kernels (``set_queue(lag=..., split=...)``)
-        is chosen."""
-        return (self.npe == 4 and not self.queued_k and self.wait_spins == 0
-                and self.n_elements <= self.TWO_PASS_K_ELEMENTS)
+        """The same for the tangent sweeps (Tet10, and FP32 ones of Tet4) of meshes up to
+        ``TWO_PASS_K_ELEMENTS``: until a lag of the K queue or one of its kernels
+        (``set_queue(lag=..., split=...)``) is chosen."""
+        return not self.queued_k and self.wait_spins == 0 and self.n_elements <= self.TWO_PASS_K_ELEMENTS
 
     def set_two_pass(self, f: bool = True, k: bool = True) -> None:
         """Back to the two-pass sweeps (without and with a tangent) after ``set_queue``; a
@@ -260,7 +261,7 @@ class MeshPattern:
         warp-specialised kernel (``split``; the mixed kernel otherwise).
 
         With ``lag_f``, the sweeps without a tangent run the queued kernel instead of two
-        passes; with ``lag`` or ``split``, the FP32 tangent sweeps (``set_two_pass`` goes back).
+        passes; with ``lag`` or ``split``, the tangent sweeps too (``set_two_pass`` goes back).
         Rebuilds the task queues when a lag changes; a workspace sized for the old values must
         be re-queried (``psx_work_bytes``) afterwards.
         """

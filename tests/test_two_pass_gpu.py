@@ -1,4 +1,4 @@
-"""Tet4 sweeps in two passes against the queued kernels (GPU).
+"""Sweeps in two passes against the queued kernels (GPU).
 
 Same element code, tile records and association: f, K.v, dynamic relaxation, the adjoint and
 the FP32 tangents must be equal bit for bit.  Meshes at the edges of the tiles: one element, a last tile of
@@ -47,7 +47,7 @@ def _pair(mesh, precision):
     mu = np.random.default_rng(4).uniform(1e3, 5e3, mesh.n_elements)
     field = NeoHookeanField(mu, 20.0 * mu, mass_density=900.0)
     a, b = (GPUAssembler(mesh.nodes, mesh.elements, field, precision=precision) for _ in range(2))
-    b.set_queue(lag_f=b.pattern.lag_f, split=True)
+    b.set_queue(lag=b.pattern.lag, lag_f=b.pattern.lag_f, split=True)
     way = lambda s: (s.dev["plan"].two_pass, s.dev["plan"].two_pass_k)  # noqa: E731
     assert way(a) == (1, 1) and way(b) == (0, 0)
     X = mesh.nodes
@@ -76,6 +76,25 @@ def test_two_pass_sweeps_equal_the_queued_kernels(name, precision):
         for _ in range(3):
             s.dr_step(u, v, torch.full_like(v, 1e-6), x, vel, 0.9, 1.9, 1.0, r_out=r)
         yield from (("x", x), ("vel", vel), ("r", r))
+
+    for (what, x), (_, y) in zip(sweeps(a), sweeps(b)):
+        assert torch.equal(x, y), what
+    assert a.status_counts() == (0, 0, -1, 0)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32-mixed"])
+@pytest.mark.parametrize("name", ["one element", "33 elements", "ragged box", "shuffled box"])
+def test_tet10_two_pass_sweeps_equal_the_queued_kernel(name, precision):
+    # tiles of 8 elements: 1, 4 x 8 + 1, ...; every sum has the same terms in the same order
+    mesh = meshgen.tet4_to_tet10(MESHES[name]())
+    a, b, u, v = _pair(mesh, precision)
+
+    def sweeps(s):
+        yield "f", s.assemble(u, want_k=False)[0]
+        yield from zip(("f of f+K", "K of f+K"), s.assemble(u))
+        yield "K", s.assemble(u, want_f=False)[1]
+        yield "mass", s.assemble(None, mass=True)[1]
+        yield "linear", s.assemble(None, linear=True)[1]
 
     for (what, x), (_, y) in zip(sweeps(a), sweeps(b)):
         assert torch.equal(x, y), what

@@ -1,5 +1,5 @@
-"""Which way the Tet4 sweeps run (CPU): two passes by default, the queued kernels once a shape
-of their queue is chosen or its waits are limited, and for FP32 tangents of large meshes."""
+"""Which way the sweeps run (CPU): two passes by default, the queued kernels once a shape
+of their queue is chosen or its waits are limited, and for tangents of large meshes."""
 from __future__ import annotations
 
 from psierra_b200 import meshgen
@@ -31,5 +31,10 @@ def test_choices():
     p.set_two_pass()
     assert way() == (1, 0)
     t10 = meshgen.tet4_to_tet10(m)
-    st = MeshPattern(t10.elements, t10.n_nodes).device("cpu")["plan"]
-    assert (st.two_pass, st.two_pass_k) == (0, 0)
+    p = MeshPattern(t10.elements, t10.n_nodes)
+    st = p.device("cpu")["plan"]
+    assert way() == (1, 1)
+    p.set_queue(lag=3)
+    assert way() == (1, 0)
+    p.set_queue(lag_f=3)
+    assert way() == (0, 0)
