@@ -170,8 +170,22 @@ typedef struct psx_plan {
   int32_t two_pass;
   int32_t two_pass_k;       /* the same for the FP32 tangent sweeps of psx_tet4_assemble[_effective]
                                and all tangent sweeps of psx_tet10_assemble */
-  int32_t reserved0;        /* 0 */
+  /* Bit 0 (FP64) and bit 1 (FP32): f + K and K-only sweeps of psx_tet4_assemble run in two
+     launches on point records of the whole mesh (psx_work_bytes counts them): the elements'
+     factors, then each pair's and node's blocks formed and summed from them.  They need the
+     lists of psx_point_lists.  FP64 values are the queued kernel's bit for bit; FP32 ones are
+     summed in FP64, per element instead of per element tile. */
+  int32_t two_pass_p;
+  const int32_t* pair_base; /* device, ceil(n_pairs / 32) + 1: where the lists of each 32 pairs start */
+  int32_t* pair_list;       /* device, pair_base[last]: e * 16 + a * 4 + b, a local node of the rows; -1 = none */
+  const int32_t* node_base; /* device, ceil(n_nodes / 32) + 1 */
+  int32_t* node_list;       /* device, node_base[last]: e * 16 + a; -1 = none */
 } psx_plan_t;
+
+/* Fill pair_list and node_list (device) from pair_ptr, pair_src, node_ptr, node_src: entry k of
+ * item 32 w + l of the list at base[w] + 32 k + l, base[w + 1] - base[w] = 32 times the longest
+ * of the 32 lists. */
+int psx_point_lists(const psx_plan_t* plan, void* stream);
 
 /* n_pairs = (sum deg - N) / 2 and the pair_src length E * npe (npe - 1) / 2 (host). */
 int psx_plan_count(const int64_t* conn, int64_t E, int npe, int64_t N, const int32_t* nbr_ptr,

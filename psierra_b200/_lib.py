@@ -51,6 +51,7 @@ SIGNATURES: dict[str, list] = {
     "psx_plan_fill": [_p, _i64, _i32, _i64, _p, _p, _i64, _p, _p, _p, _p, _p, _p, _p, _p, _p],
     "psx_task_count": [_p, _i32, _i32, _i32, _i32, _p],
     "psx_task_fill": [_p, _i32, _i32, _i32, _i32, _p, _p],
+    "psx_point_lists": [_p, _p],
     "psx_work_bytes": [_p, _i32, _p, _p],
     "psx_tet4_assemble": [_p, _p, _p, _p, _p, _f64, _f64, _f64, _i32, _i32, _p, _p, _p, _i64, _p, _p],
     "psx_tet4_kv": [_p, _p, _p, _p, _p, _f64, _f64, _i32, _p, _p, _p, _i64, _p, _p],
@@ -135,7 +136,11 @@ class PlanStruct(ctypes.Structure):
         ("wait_spins", ctypes.c_int32),
         ("two_pass", ctypes.c_int32),
         ("two_pass_k", ctypes.c_int32),
-        ("reserved0", ctypes.c_int32),
+        ("two_pass_p", ctypes.c_int32),
+        ("pair_base", ctypes.c_void_p),
+        ("pair_list", ctypes.c_void_p),
+        ("node_base", ctypes.c_void_p),
+        ("node_list", ctypes.c_void_p),
     ]
 
 

@@ -103,16 +103,15 @@ class GPUAssembler:
     # ------------------------------------------------------------------ workspace
     def launches_per_call(self, precision: str | None = None) -> int:
         """Kernel launches of one assemble() of f and K: one persistent kernel, or two passes."""
-        two = self.pattern.two_pass_k and (self.npe == 10 or (precision or self.precision) == "fp32-mixed")
-        return 2 if two else 1
+        return 2 if self.pattern.tangent_in_two_passes(precision or self.precision) else 1
 
     def set_queue(self, lag: int | None = None, blocks_per_sm: int | None = None,
                   ring_slack: int | None = None, lag_f: int | None = None, split: bool | None = None) -> None:
         """Launch shape of the persistent kernel (see ``MeshPattern.set_queue``)."""
         p = self.pattern
-        old = (p.lag, p.lag_f, p.ring_slack, p.two_pass, p.two_pass_k)
+        old = (p.lag, p.lag_f, p.ring_slack, p.two_pass, p.two_pass_k, p.point_precisions)
         p.set_queue(lag=lag, blocks_per_sm=blocks_per_sm, ring_slack=ring_slack, lag_f=lag_f, split=split)
-        if (p.lag, p.lag_f, p.ring_slack, p.two_pass, p.two_pass_k) != old:
+        if (p.lag, p.lag_f, p.ring_slack, p.two_pass, p.two_pass_k, p.point_precisions) != old:
             self._work.clear()  # the records are sized by the lag, the slack and the passes
 
     def set_two_pass(self, f: bool = True, k: bool = True) -> None:

@@ -100,7 +100,7 @@ def tune(asm, u: torch.Tensor, precision: str | None = None, want_f: bool = True
     if hasattr(asm, "set_two_pass"):
         # sweeps that also run in two passes, without a queue: keep the faster way
         asm.set_two_pass(f=not want_k, k=want_k)
-        if (asm.pattern.two_pass_k and (asm.npe == 10 or prec == "fp32-mixed") if want_k else asm.pattern.two_pass) and \
+        if (asm.pattern.tangent_in_two_passes(prec) if want_k else asm.pattern.two_pass) and \
                 _time(asm, u, prec, want_f, want_k, f, k, reps) < table[best]:
             entry = best + (True,)
         else:

@@ -202,6 +202,21 @@ __device__ __forceinline__ Quad ld_quad_nc(const double* p) {  // memory no thre
   asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(q.x), "=d"(q.y), "=d"(q.z), "=d"(q.w) : "l"(p));
   return q;
 }
+__device__ __forceinline__ void st_quad(double* p, const Quad& q) {
+  asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(q.x), "d"(q.y), "d"(q.z), "d"(q.w) : "memory");
+}
+__device__ __forceinline__ void st_oct(float* p, float a, float b, float c, float d, float e, float f, float g, float h) {
+  asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d),
+               "f"(e), "f"(f), "f"(g), "f"(h)
+               : "memory");
+}
+// Eight floats at once, as ld_quad_nc.
+__device__ __forceinline__ void ld_oct_nc(const float* p, float& a, float& b, float& c, float& d, float& e, float& f,
+                                          float& g, float& h) {
+  asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=f"(a), "=f"(b), "=f"(c), "=f"(d), "=f"(e), "=f"(f), "=f"(g), "=f"(h)
+               : "l"(p));
+}
 __device__ __forceinline__ Quad ld_quad(const double* p) {
   Quad q;
   asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(q.x), "=d"(q.y), "=d"(q.z), "=d"(q.w) : "l"(p));

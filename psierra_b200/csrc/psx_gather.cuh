@@ -819,6 +819,13 @@ inline int work_layout(const psx_plan_t* P, int precision, void* work, WorkLayou
     fbytes = up(ring_elems * kF * 8);
   }
   W->total_bytes = (int64_t)W->counter_bytes + kbytes + fbytes;
+  if (P->npe == 4 && queue_k && (P->two_pass_p & (precision == PSX_FP64 ? 1 : 2))) {
+    // point records (run_points): 32 values per element, then f per element (FP64) or tile
+    const int64_t cn4 = (P->tile_cap_nodes + 3) / 4 * 4;
+    const int64_t f = precision == PSX_FP64 ? P->n_elements * 96 : (P->n_elements + P->tile - 1) / P->tile * 24 * cn4;
+    const int64_t points = (int64_t)W->counter_bytes + P->n_elements * 32 * kt + f;
+    if (points > W->total_bytes) W->total_bytes = points;
+  }
   W->counters = nullptr;
   W->krec = nullptr;
   W->frec = nullptr;

@@ -264,6 +264,7 @@ __device__ __forceinline__ void tet4_element(const Tet4Args& A, int64_t e, const
         h[b][k] = xmul(tc.hb, p[b][k]);
         y[b][k] = xmul(tc.c, q[b][k]);
       }
+    constexpr bool kPoint = sizeof(KT) == 8 && !kEff && !kLinear;
     const int gid[4] = {cn.x, cn.y, cn.z, cn.w};
     int slot = 0;
 #pragma unroll
@@ -272,6 +273,8 @@ __device__ __forceinline__ void tet4_element(const Tet4Args& A, int64_t e, const
       for (int b = a; b < 4; ++b) {
         const KT gg = xdot3(gk[a][0], gk[b][0], gk[a][1], gk[b][1], gk[a][2], gk[b][2]);
         KT s = xmul(tc.phi, gg);
+        // as the point records form it (point_block): c = -2/3 phi
+        if constexpr (kPoint) s = xmul((KT)-1.5, xdot3(p[a][0], y[b][0], p[a][1], y[b][1], p[a][2], y[b][2]));
         if constexpr (kEff) s = xadd(s, xfma(e_mu, gg, xmul(e_mass, a == b ? (KT)2 : (KT)1)));
         KT v[9];
 #pragma unroll
@@ -688,6 +691,31 @@ bool split_usable() {
   return s_regs == kSplitLaunchRegs;
 }
 
+// Contribution lists of the point records (psx_point_lists): the lists of 32 consecutive items
+// side by side, entry k of lane l at base + 32 k + l, -1 past an item's end.  A pair's entry is
+// e * 16 + a * 4 + b with a the local node of the row block, a node's e * 16 + a.
+__global__ void point_lists_kernel(const int32_t* __restrict__ conn, const int32_t* __restrict__ ptr,
+                                   const int32_t* __restrict__ src, const int32_t* __restrict__ base, int32_t n,
+                                   bool pairs, int32_t* __restrict__ list) {
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i >= (n + 31LL) / 32 * 32) return;
+  int32_t s = i < n ? ptr[i] : 0;
+  const int32_t s1 = i < n ? ptr[i + 1] : 0;
+  for (int32_t k = base[i >> 5] + (int32_t)(i & 31); k < base[(i >> 5) + 1]; k += 32, ++s) {
+    int32_t c = -1;
+    if (s < s1) {
+      c = src[s];
+      if (pairs) {
+        const int32_t e = c >> 6, slot = c & 63;
+        const int a = (0x940 >> (2 * slot)) & 3, b = (0xFB9 >> (2 * slot)) & 3;  // 01 02 03 12 13 23
+        const bool swap = conn[4 * (int64_t)e + a] > conn[4 * (int64_t)e + b];
+        c = e * 16 + (swap ? b * 4 + a : a * 4 + b);
+      }
+    }
+    list[k] = c;
+  }
+}
+
 __global__ void tet4_dets_kernel(const int32_t* __restrict__ conn, const double* __restrict__ X,
                                  const double* __restrict__ U, int64_t e, double* out2) {
   const int4 cn = reinterpret_cast<const int4*>(conn)[e];
@@ -709,6 +737,259 @@ __global__ void tet4_dets_kernel(const int32_t* __restrict__ conn, const double*
   }
 }
 
+// ---- tangents from point records --------------------------------------------------------
+// f + K and K-only sweeps in two launches with less memory between them than element blocks
+// take: pass 1 stores an element's factors (per node p, A, y = c q and hb: 256 bytes in FP64,
+// 128 in FP32, against 832 bytes of FP64 blocks), pass 2 forms each 3x3 block where it is
+// summed, one thread per pair / node over the elements in ascending order.  phi g_a.g_b
+// follows from the factors as -3/2 p_a.y_b (p = F^-T g, q = F g, c = -2/3 phi), so the
+// geometry isn't stored; the queued FP64 kernel forms it the same way and gives the same bits.
+// FP32 factors are rounded once from FP64 ones and the blocks summed in FP64, at no cost here:
+// the error of K against the FP64 sweep is 3.5e-8 of its norm (5.2e-8 from the queue, 7.5e-8
+// with FP32 sums in element order).  The FP32 f triples go through tile records
+// (22 bytes per element), the FP64 ones are stored per element, as the queue sums them.
+// Measured on Kuhn cubes, us, f + K (K):
+//   elements    FP64 queue     points         FP32 queue / tiles   points
+//     384,000    203 (185)     118 (107)         94  (84)           80  (68)
+//   1,053,696    520 (476)     283 (241)        235 (219)          180 (152)
+//   3,072,000   1564 (1420)    775 (691)        634 (584)          485 (405)
+// Pass 1 takes 179 of the last 485 us (FP64 chain at 20 warps per SM, 45% of issue slots),
+// pass 2 the rest: gathered 32-byte loads (62M sectors through L1, 1.0 GB of DRAM traffic,
+// 3.1 TB/s).  What made the difference there: node blocks spread among the pair blocks, so
+// that both read a record while it is in L2 (1.05M elements, FP64: 377 -> 317 us); planes
+// instead of one 256-byte record per element (480 -> 393); lists side by side per warp with
+// the orientation in them, read one batch ahead (FP32, 3.07M: 546 -> 488).
+struct PointArgs {
+  const int4* pair_info;
+  const int32_t* pair_base;
+  const int32_t* pair_list;
+  const int4* node_info;
+  const int32_t* node_base;
+  const int32_t* node_list;
+  int32_t n_pairs, n_nodes;
+  int64_t n_elements;
+};
+// Of each node, in planes over the elements: 32 bytes (FP32) or two times 32 (FP64).  f of the
+// FP64 sweep: 12 planes of doubles (four of 32 bytes: 317 us at 304, 1.05M elements).
+template <typename KT>
+struct PointRec {
+  KT p[3], A, y[3], hb;
+};
+template <typename KT>
+__device__ __forceinline__ void st_point(KT* krec, int64_t n, int64_t e, int a, const PointRec<KT>& r) {
+  if constexpr (sizeof(KT) == 8) {
+    st_quad(krec + ((2 * a) * n + e) * 4, Quad{r.p[0], r.p[1], r.p[2], r.A});
+    st_quad(krec + ((2 * a + 1) * n + e) * 4, Quad{r.y[0], r.y[1], r.y[2], r.hb});
+  } else {
+    st_oct(krec + (a * n + e) * 8, r.p[0], r.p[1], r.p[2], r.A, r.y[0], r.y[1], r.y[2], r.hb);
+  }
+}
+template <typename KT>
+__device__ __forceinline__ PointRec<KT> ld_point(const KT* krec, int64_t n, int64_t e, int a) {
+  PointRec<KT> r;
+  if constexpr (sizeof(KT) == 8) {
+    const Quad x = ld_quad_nc(krec + ((2 * a) * n + e) * 4), y = ld_quad_nc(krec + ((2 * a + 1) * n + e) * 4);
+    r.p[0] = x.x; r.p[1] = x.y; r.p[2] = x.z; r.A = x.w;
+    r.y[0] = y.x; r.y[1] = y.y; r.y[2] = y.z; r.hb = y.w;
+  } else {
+    ld_oct_nc(krec + (a * n + e) * 8, r.p[0], r.p[1], r.p[2], r.A, r.y[0], r.y[1], r.y[2], r.hb);
+  }
+  return r;
+}
+
+template <typename KT, int MODE>
+__device__ __forceinline__ void points_element(const Tet4Args& A, int64_t e, int64_t n_el, KT* __restrict__ krec,
+                                               double* __restrict__ frec) {
+  const int4 cn = __ldg(reinterpret_cast<const int4*>(A.conn) + e);
+  double Xn[4][3], Un[4][3];
+  load_nodes(A.X, cn, Xn);
+  load_nodes(A.U, cn, Un);
+  Tet4Geom G;
+  tet4_geometry(Xn, G);
+  if (!(G.detD > 0.0)) flag_bad_element(A.st, e, true);
+  const double mu = A.mu_e ? A.mu_e[e] : A.mu0;
+  const double kappa = A.kappa_e ? A.kappa_e[e] : A.kappa0;
+  double l[3][3];
+  tet4_grad(Un, G, l);
+  PointState ps;
+  neohookean_point(l, mu, kappa, ps);
+  if (G.detD > 0.0 && ps.Jm1 <= -1.0) flag_bad_element(A.st, e, false);
+  if constexpr ((MODE & PSX_WANT_F) != 0) {
+    double fr[12];
+    tet4_force(ps, G, fr);
+#pragma unroll
+    for (int j = 0; j < 12; ++j) frec[sizeof(KT) == 4 ? j : j * n_el + e] = fr[j];
+  }
+  const TangentCoef<double> tc = tangent_coef<double>(ps, kappa, G.V);
+  double p[4][3], q[4][3];
+  tet4_pq<double>(ps, G.g, p, q);
+#pragma unroll
+  for (int a = 0; a < 4; ++a) {
+    PointRec<KT> r;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      r.p[k] = (KT)p[a][k];
+      r.y[k] = (KT)dmul(tc.c, q[a][k]);
+    }
+    r.A = (KT)tc.A;
+    r.hb = (KT)tc.hb;
+    st_point(krec, n_el, e, a, r);
+  }
+}
+
+template <typename KT, int MODE>
+__global__ void __launch_bounds__(kThreads, sizeof(KT) == 8 ? 4 : 5)
+tet4_points_kernel(Tet4Args A, GatherArgs g, int64_t n_el, KT* __restrict__ krec, double* __restrict__ frec) {
+  constexpr bool kWantF = (MODE & PSX_WANT_F) != 0, kTileF = kWantF && sizeof(KT) == 4;
+  int64_t e = blockIdx.x * (int64_t)kThreads + threadIdx.x, t = 0;
+  bool active = e < n_el;
+  __shared__ __align__(16) double s_f[kTileF ? kThreads * kFStride : 2];
+  __shared__ __align__(16) unsigned char s_meta[kTileF ? kThreads / 32 * kMetaBytes : 16];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  double* fst = s_f + (kTileF ? warp * 32 * kFStride : 0);
+  unsigned char* lst = s_meta + (kTileF ? warp * kMetaBytes : 0);
+  if constexpr (kTileF) {
+    t = blockIdx.x * (int64_t)(kThreads / 32) + warp;
+    if (t * g.tile >= n_el) return;
+    e = t * g.tile + lane;
+    active = lane < g.tile && e < n_el;
+    tile_meta_prefetch<false>(g, t, lst);
+  }
+  if (active) points_element<KT, MODE>(A, e, n_el, krec, kTileF ? fst + kFStride * lane : frec);
+  if constexpr (kTileF) {
+    cp_async_wait_all();
+    __syncwarp();
+    tile_reduce<false, true, false>(g, t, lst, nullptr, fst, nullptr, frec);
+  }
+}
+// Records in flight per thread: two per pair (3: 289 us at 283, FP64, 1.05M elements), per
+// node four, or two in FP64 with f (4: 289 at 283; K alone 254 with 2, 241 with 4).
+template <typename KT, int MODE>
+__global__ void __launch_bounds__(kItemThreads)
+tet4_point_items_kernel(PointArgs g, GatherArgs gt, const KT* __restrict__ krec, const double* __restrict__ frec,
+                        KT* __restrict__ k_out, double* __restrict__ f_out) {
+  constexpr bool kWantF = (MODE & PSX_WANT_F) != 0 && sizeof(KT) == 8, kTileF = (MODE & PSX_WANT_F) != 0 && !kWantF;
+  constexpr int kPairs = 2, kNodes = kWantF ? 2 : 4;
+  const int64_t n_el = g.n_elements;
+  // blocks of nodes spread evenly among the blocks of pairs
+  const int32_t nb = (g.n_nodes + kItemThreads - 1) / kItemThreads;
+  const int32_t nodes_before = (int32_t)((int64_t)blockIdx.x * nb / gridDim.x);
+  const bool node_block = (int32_t)((int64_t)(blockIdx.x + 1) * nb / gridDim.x) > nodes_before;
+  if (!node_block) {
+    const int32_t i = (blockIdx.x - nodes_before) * kItemThreads + threadIdx.x;
+    if (i >= g.n_pairs) return;
+    const int4 info = __ldg(g.pair_info + i);
+    const int32_t s1 = __ldg(g.pair_base + (i >> 5) + 1);
+    double acc[9];
+#pragma unroll
+    for (int j = 0; j < 9; ++j) acc[j] = 0.0;
+    int32_t s = __ldg(g.pair_base + (i >> 5)) + (i & 31), nxt[kPairs];
+#pragma unroll
+    for (int u = 0; u < kPairs; ++u) nxt[u] = s + 32 * u < s1 ? __ldg(g.pair_list + s + 32 * u) : -1;
+    for (; s < s1; s += 32 * kPairs) {
+      PointRec<KT> ra[kPairs], rb[kPairs];
+      int32_t c[kPairs];
+#pragma unroll
+      for (int u = 0; u < kPairs; ++u) {
+        c[u] = nxt[u];
+        nxt[u] = s + 32 * (kPairs + u) < s1 ? __ldg(g.pair_list + s + 32 * (kPairs + u)) : -1;
+      }
+#pragma unroll
+      for (int u = 0; u < kPairs; ++u)
+        if (c[u] >= 0) {
+          const int a = (c[u] >> 2) & 3, b = c[u] & 3;
+          ra[u] = ld_point(krec, n_el, c[u] >> 4, min(a, b));
+          rb[u] = ld_point(krec, n_el, c[u] >> 4, max(a, b));
+        }
+#pragma unroll
+      for (int u = 0; u < kPairs; ++u)
+        if (c[u] >= 0) {
+          const bool swap = ((c[u] >> 2) & 3) > (c[u] & 3);
+          KT v[9];
+          point_block(ra[u].p, ra[u].y, rb[u].p, rb[u].y, ra[u].A, ra[u].hb, v);
+#pragma unroll
+          for (int k = 0; k < 3; ++k)
+#pragma unroll
+            for (int m = 0; m < 3; ++m) acc[3 * k + m] += swap ? v[3 * m + k] : v[3 * k + m];
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < 3; ++k) store3(k_out + info.x + (int64_t)info.y * k, (KT)acc[3 * k], (KT)acc[3 * k + 1], (KT)acc[3 * k + 2]);
+#pragma unroll
+    for (int m = 0; m < 3; ++m) store3(k_out + info.z + (int64_t)info.w * m, (KT)acc[m], (KT)acc[3 + m], (KT)acc[6 + m]);
+  } else {
+    const int32_t n = nodes_before * kItemThreads + threadIdx.x;
+    if (n >= g.n_nodes) return;
+    const int4 info = __ldg(g.node_info + n);
+    const int32_t s1 = __ldg(g.node_base + (n >> 5) + 1);
+    double acc[6] = {0, 0, 0, 0, 0, 0}, fa[3] = {0, 0, 0};
+    int32_t s = __ldg(g.node_base + (n >> 5)) + (n & 31), nxt[kNodes];
+#pragma unroll
+    for (int u = 0; u < kNodes; ++u) nxt[u] = s + 32 * u < s1 ? __ldg(g.node_list + s + 32 * u) : -1;
+    for (; s < s1; s += 32 * kNodes) {
+      PointRec<KT> ra[kNodes];
+      double fv[kNodes][3];
+      int32_t c[kNodes];
+#pragma unroll
+      for (int u = 0; u < kNodes; ++u) {
+        c[u] = nxt[u];
+        nxt[u] = s + 32 * (kNodes + u) < s1 ? __ldg(g.node_list + s + 32 * (kNodes + u)) : -1;
+      }
+#pragma unroll
+      for (int u = 0; u < kNodes; ++u)
+        if (c[u] >= 0) {
+          const int a = c[u] & 15;
+          ra[u] = ld_point(krec, n_el, c[u] >> 4, a);
+          if constexpr (kWantF)
+#pragma unroll
+            for (int k = 0; k < 3; ++k) fv[u][k] = __ldg(frec + (3 * a + k) * n_el + (c[u] >> 4));
+        }
+#pragma unroll
+      for (int u = 0; u < kNodes; ++u)
+        if (c[u] >= 0) {
+          KT v[9];
+          point_block(ra[u].p, ra[u].y, ra[u].p, ra[u].y, ra[u].A, ra[u].hb, v);
+          acc[0] += v[0]; acc[1] += v[1]; acc[2] += v[2]; acc[3] += v[4]; acc[4] += v[5]; acc[5] += v[8];
+          if constexpr (kWantF)
+#pragma unroll
+            for (int k = 0; k < 3; ++k) fa[k] += fv[u][k];
+        }
+    }
+    if (info.y > 0) {
+      store3(k_out + info.x, (KT)acc[0], (KT)acc[1], (KT)acc[2]);
+      store3(k_out + info.x + (int64_t)info.y, (KT)acc[1], (KT)acc[3], (KT)acc[4]);
+      store3(k_out + info.x + (int64_t)info.y * 2, (KT)acc[2], (KT)acc[4], (KT)acc[5]);
+    }
+    if constexpr (kWantF) store3(f_out + 3 * (int64_t)info.z, fa[0], fa[1], fa[2]);
+    if constexpr (kTileF)
+      gather_node<double, 4, false, true, false, true, 0, false, true>(gt, node_head<true>(gt, n), nullptr, frec, nullptr, f_out);
+  }
+}
+
+template <typename KT, int MODE>
+int run_points(const psx_plan_t* P, const Tet4Args& A, const WorkLayout& W, KT* k_out, double* f_out,
+               cudaStream_t stream) {
+  constexpr bool tile_f = sizeof(KT) == 4 && (MODE & PSX_WANT_F) != 0;
+  GatherArgs gt = gather_args(P, W.ring_elems);
+  gt.ring_tile_mask = INT64_MAX;  // one tile record per tile
+  if (!P->pair_base || !P->pair_list || !P->node_base || !P->node_list || P->n_pairs + P->n_nodes > 0x7fffff00 ||
+      (tile_f && (P->tile > 32 || gt.meta_stride > kMetaBytes)))
+    return PSX_ERR_ARG;
+  KT* krec = static_cast<KT*>(W.krec);
+  double* frec = reinterpret_cast<double*>(krec + 32 * P->n_elements);
+  const int64_t per = tile_f ? kThreads / 32 * P->tile : kThreads;
+  tet4_points_kernel<KT, MODE><<<(unsigned)((P->n_elements + per - 1) / per), kThreads, 0, stream>>>(A, gt, P->n_elements, krec,
+                                                                                                    frec);
+  const PointArgs g{reinterpret_cast<const int4*>(P->pair_info), P->pair_base, P->pair_list,
+                    reinterpret_cast<const int4*>(P->node_info), P->node_base, P->node_list,
+                    (int32_t)P->n_pairs, (int32_t)P->n_nodes, P->n_elements};
+  const int64_t blocks =
+      (P->n_pairs + kItemThreads - 1) / kItemThreads + (P->n_nodes + kItemThreads - 1) / kItemThreads;
+  tet4_point_items_kernel<KT, MODE><<<(unsigned)blocks, kItemThreads, 0, stream>>>(g, gt, krec, frec, k_out, f_out);
+  PSX_CUDA_CHECK_LAUNCH();
+  return PSX_OK;
+}
+
 template <typename KT, int MODE>
 int run_tet4(const psx_plan_t* P, const Tet4Args& A, const WorkLayout& W, KT* k_out, double* f_out,
              cudaStream_t stream, const DRArgs& dr = DRArgs{}) {
@@ -717,6 +998,9 @@ int run_tet4(const psx_plan_t* P, const Tet4Args& A, const WorkLayout& W, KT* k_
   // every sweep without a tangent is faster in two passes (tet4_tiles_kernel), at all sizes
   if constexpr (!kWantK) {
     if (P->two_pass) return run_two_pass<KT, MODE>(P, A, W, nullptr, f_out, stream, dr);
+  }
+  if constexpr (kWantK && sizeof(KT) == 8 && (MODE & (PSX_LINEAR | PSX_MASS | kModeEff)) == 0) {
+    if ((P->two_pass_p & (sizeof(KT) == 8 ? 1 : 2))) return run_points<KT, MODE>(P, A, W, k_out, f_out, stream);
   }
   const GatherArgs g = gather_args(P, W.ring_elems);
   const QueueArgs Q = queue_args(P, W, kWantK);
@@ -772,6 +1056,8 @@ int run_tet4_split(const psx_plan_t* P, const Tet4Args& A, const WorkLayout& W, 
 template <int MODE>
 int run_tet4_k32(const psx_plan_t* P, const Tet4Args& A, const WorkLayout& W, float* k_out, double* f_out,
                  cudaStream_t stream) {
+  if constexpr ((MODE & (PSX_LINEAR | PSX_MASS | kModeEff)) == 0)
+    if ((P->two_pass_p & 2)) return run_points<float, MODE>(P, A, W, k_out, f_out, stream);
   if (P->two_pass_k && W.tiles) return run_two_pass<float, MODE>(P, A, W, k_out, f_out, stream, DRArgs{});
   if (P->gtasks_k && P->n_gtasks_k > 0 && W.tiles && split_usable<float, MODE>())
     return run_tet4_split<float, MODE>(P, A, W, k_out, f_out, stream);
@@ -785,6 +1071,22 @@ extern "C" size_t psx_status_bytes(void) { return sizeof(psx::Status); }
 
 extern "C" int psx_tet4_split_ready(void) {
   return psx::split_usable<float, PSX_WANT_F | PSX_WANT_K>() && psx::split_usable<float, PSX_WANT_K>() ? 1 : 0;
+}
+
+extern "C" int psx_point_lists(const psx_plan_t* plan, void* stream) {
+  if (!plan || plan->npe != 4 || !plan->conn || !plan->pair_ptr || !plan->pair_src || !plan->node_ptr ||
+      !plan->node_src || !plan->pair_base || !plan->pair_list || !plan->node_base || !plan->node_list ||
+      plan->n_nodes <= 0 || plan->n_nodes > 0x7fffff00 || plan->n_pairs < 0 || plan->n_pairs > 0x7fffff00)
+    return PSX_ERR_ARG;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  const int32_t np = (int32_t)plan->n_pairs, nn = (int32_t)plan->n_nodes;
+  if (np > 0)
+    psx::point_lists_kernel<<<(unsigned)((np + 255LL) / 256), 256, 0, s>>>(plan->conn, plan->pair_ptr, plan->pair_src,
+                                                                           plan->pair_base, np, true, plan->pair_list);
+  psx::point_lists_kernel<<<(unsigned)((nn + 255LL) / 256), 256, 0, s>>>(plan->conn, plan->node_ptr, plan->node_src,
+                                                                         plan->node_base, nn, false, plan->node_list);
+  PSX_CUDA_CHECK_LAUNCH();
+  return PSX_OK;
 }
 
 extern "C" int psx_work_bytes(const psx_plan_t* plan, int precision, int64_t* ring_elems, int64_t* bytes) {

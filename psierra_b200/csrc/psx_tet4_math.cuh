@@ -119,6 +119,27 @@ __device__ __forceinline__ void tet4_pq(const PointState& ps, const KT gk[4][3],
     }
 }
 
+// Block K_ab = A p_a p_b^T + hb p_b p_a^T + p_a y_b^T + y_a p_b^T + phi (g_a.g_b) I of an element
+// (y = c q; phi g_a.g_b = -3/2 p_a.y_b), in the association of tet4_element.
+template <typename KT>
+__device__ __forceinline__ void point_block(const KT pa[3], const KT ya[3], const KT pb[3], const KT yb[3], KT A, KT hb,
+                                            KT v[9]) {
+  const KT s = xmul((KT)-1.5, xdot3(pa[0], yb[0], pa[1], yb[1], pa[2], yb[2]));
+  KT w[3], h[3];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    w[k] = xfma(A, pb[k], yb[k]);
+    h[k] = xmul(hb, pa[k]);
+  }
+#pragma unroll
+  for (int k = 0; k < 3; ++k)
+#pragma unroll
+    for (int m = 0; m < 3; ++m) {
+      const KT last = k == m ? xfma(ya[k], pb[m], s) : xmul(ya[k], pb[m]);
+      v[3 * k + m] = xfma(pa[k], w[m], xfma(pb[k], h[m], last));
+    }
+}
+
 // Sums over the element's nodes of a vector v that the product K_e v and the adjoint use:
 // alpha = sum_b w_b.v_b (w = A p + c q), beta = sum_b p_b.v_b, Pv = sum_b p_b v_b^T,
 // Gv = sum_b g_b v_b^T.

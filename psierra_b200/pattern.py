@@ -173,9 +173,35 @@ class MeshPattern:
                     setattr(st, k, d[k].data_ptr())
                 st.tile_cap_pairs, st.tile_cap_nodes = int(h["tile_caps"][0]), int(h["tile_caps"][1])
             d["plan"] = st
+            if self.npe == 4 and d["device"].type == "cuda" and self.n_elements <= self.POINT_ELEMENTS:
+                with torch.cuda.device(d["device"]):
+                    self._build_point_lists(d)
             self._build_tasks(d)
             self._dev = d
         return self._dev
+
+    def _build_point_lists(self, d: dict) -> None:
+        """The lists of the point records (``psx_point_lists``), on the device."""
+        import torch
+
+        st, new = d["plan"], {}
+        for key in ("pair", "node"):
+            n = d[key + "_ptr"].numel() - 1
+            width = torch.zeros((n + 31) // 32 * 32, dtype=torch.int32, device=d["device"])
+            width[:n] = d[key + "_ptr"].diff()
+            ends = (width.view(-1, 32).amax(1).long() * 32).cumsum(0)
+            size = int(ends[-1]) if n else 0
+            if size > 4 * d[key + "_src"].numel() + 4096:  # a few long lists, mostly padding: the queue
+                return
+            base = torch.zeros(ends.numel() + 1, dtype=torch.int32, device=d["device"])
+            base[1:] = ends
+            new[key + "_base"], new[key + "_list"] = base, torch.empty(max(size, 1), dtype=torch.int32, device=d["device"])
+        for k, v in new.items():
+            setattr(st, k, v.data_ptr())
+        stream = torch.cuda.current_stream()
+        check(lib().psx_point_lists(ctypes.byref(st), stream.cuda_stream), "psx_point_lists")
+        stream.synchronize()  # sweeps may run on any stream
+        d.update(new)
 
     def _build_tasks(self, d: dict) -> None:
         """(Re)build the element/gather task queues of the plan in ``d`` for the current lag."""
@@ -211,6 +237,7 @@ class MeshPattern:
         st = d["plan"]
         on = self.split and d.get("n_gtasks_k", 0) > 0
         st.two_pass, st.two_pass_k = int(self.two_pass), int(self.two_pass_k)
+        st.two_pass_p = self.point_precisions if "pair_list" in d else 0
         st.n_gtasks_k = d["n_gtasks_k"] if on else 0
         st.gtasks_k = d["gtasks_k"].data_ptr() if on else None
 
@@ -234,6 +261,28 @@ class MeshPattern:
         ``TWO_PASS_K_ELEMENTS``: until a lag of the K queue or one of its kernels
         (``set_queue(lag=..., split=...)``) is chosen."""
         return not self.queued_k and self.wait_spins == 0 and self.n_elements <= self.TWO_PASS_K_ELEMENTS
+
+    # Largest mesh (elements) on point records, and where they start in FP32.  At the upper end
+    # they hold 3.0 GB (FP64); the queue's ring does not grow with the mesh.  f + K on Kuhn
+    # cubes, us, points / queue (FP64) or the shorter of queue and two passes (FP32): FP64 384
+    # elements 13 / 18, 48,000 26 / 42, 384,000 112 / 202, 3,072,000 775 / 1564, same bits; FP32
+    # 48,000 18 / 15, 162,000 34 / 34, 235,824 47 / 51, 384,000 73 / 89, 3,072,000 480 / 634.
+    # FP32 sums are associated differently there, so one mesh's bits depend on its schedule.
+    POINT_ELEMENTS = 1 << 23
+    POINT_ELEMENTS_FP32 = 1 << 18
+
+    @property
+    def point_precisions(self) -> int:
+        """Tet4 f + K and K-only sweeps from point records (bit 0: FP64, bit 1: FP32), chosen
+        as ``two_pass_k``."""
+        if self.npe != 4 or self.queued_k or self.wait_spins or self.n_elements > self.POINT_ELEMENTS:
+            return 0
+        return 3 if self.n_elements > self.POINT_ELEMENTS_FP32 else 1
+
+    def tangent_in_two_passes(self, precision: str) -> bool:
+        """Whether f + K and K-only sweeps run in two launches (else in one persistent one)."""
+        points = self._dev is not None and self._dev["plan"].two_pass_p & (1 if precision == "fp64" else 2)
+        return bool(points) or (self.two_pass_k and (self.npe == 10 or precision == "fp32-mixed"))
 
     def set_two_pass(self, f: bool = True, k: bool = True) -> None:
         """Back to the two-pass sweeps (without and with a tangent) after ``set_queue``; a

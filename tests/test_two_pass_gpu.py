@@ -39,7 +39,7 @@ MESHES = {
     "ragged box": lambda: meshgen.box_tet4(1.0, 0.3, 0.5, 7, 3, 5),
     "shuffled box": lambda: _shuffled(meshgen.box_tet4(1.0, 1.0, 1.0, 11, 12, 13), 3),
     "uneven beams": lambda: meshgen.concat_meshes([c.mesh for c in meshgen.beam_batch(n=12, target_tets=60000, seed=3)])[0],
-    "cube 44": lambda: meshgen.box_tet4(1.0, 1.0, 1.0, 44, 44, 44),
+    "cube 34": lambda: meshgen.box_tet4(1.0, 1.0, 1.0, 34, 34, 34),
 }
 
 
@@ -102,7 +102,7 @@ def test_tet10_two_pass_sweeps_equal_the_queued_kernel(name, precision):
 
 
 def test_workspace_follows_the_way_the_sweeps_run():
-    a, b, u, v = _pair(MESHES["cube 44"](), "fp64")
+    a, b, u, v = _pair(MESHES["cube 34"](), "fp64")
     y = a.kv(u, v).clone()
     a.set_queue(lag_f=2, ring_slack=6)
     assert torch.equal(a.kv(u, v), y)
@@ -127,15 +127,67 @@ def test_larger_meshes_queue_their_fp32_tangent(monkeypatch):
     assert b.dev["plan"].two_pass_k == 1 and torch.equal(b.assemble(u)[1], k)
 
 
+@pytest.mark.parametrize("name", list(MESHES))
+def test_fp32_point_records(name, monkeypatch):
+    # f: the tile records' bits.  K: factors rounded once to FP32, about 12 roundings of terms
+    # that sum to a few times the largest entry: 5e-6 of it
+    from psierra_b200.pattern import MeshPattern
+
+    monkeypatch.setattr(MeshPattern, "POINT_ELEMENTS_FP32", 0)
+    a, b, u, v = _pair(MESHES[name](), "fp32-mixed")
+    assert a.dev["plan"].two_pass_p == 3 and b.dev["plan"].two_pass_p == 0
+    f, k = a.assemble(u)
+    assert torch.equal(f, b.assemble(u)[0])
+    k64 = b.assemble(u, precision="fp64")[1]
+    assert float((k.double() - k64).abs().max()) <= 5e-6 * float(k64.abs().max())
+    assert torch.equal(a.assemble(u, want_f=False)[1], k)
+    assert torch.equal(a.assemble(u, precision="fp64")[1], k64)
+    assert a.status_counts() == (0, 0, -1, 0)
+
+
+def test_point_records_report_bad_elements():
+    a, b, u, v = _pair(MESHES["ragged box"](), "fp64")
+    x = u.view(-1, 3).clone()
+    x[5] -= 40.0  # inverts elements around the node
+    for s in (a, b):
+        with pytest.raises(ValueError, match="inversion"):
+            s.assemble(x)
+    assert a.status_counts() == b.status_counts()
+
+
+def test_lists_that_would_be_mostly_padding_stay_queued():
+    # fans: two nodes in all 120 elements, so the 32 lists beside them would be padded to that
+    n = 120
+    ang = np.linspace(0.0, 6.0, n + 1)
+    rim = np.stack([np.cos(ang), np.sin(ang), 0.0 * ang], axis=1)
+    fan = np.vstack([[0.0, 0.0, 0.0], [0.0, 0.0, 1.0], rim])
+    el = np.array([[0, 2 + i, 3 + i, 1] for i in range(n)])
+    nodes = np.vstack([fan + [3.0 * j, 0.0, 0.0] for j in range(6)])
+    el = np.vstack([el + j * len(fan) for j in range(6)])
+    mu = np.full(len(el), 1e3)
+    a = GPUAssembler(nodes, el, NeoHookeanField(mu, 20.0 * mu))
+    b = GPUAssembler(nodes, el, NeoHookeanField(mu, 20.0 * mu))
+    b.set_queue(lag=b.pattern.lag)
+    assert a.dev["plan"].two_pass_p == 0
+    u = torch.from_numpy(1e-3 * nodes[:, [1, 2, 0]].reshape(-1)).to(DEV)
+    assert torch.equal(a.assemble(u)[1], b.assemble(u)[1])
+
+
 def test_captured_in_a_graph():
     a, b, u, v = _pair(MESHES["ragged box"](), "fp64")
-    y = b.kv(u, v)
-    out = torch.empty_like(y)
-    a.kv(u, v, y_out=out, check_status=False)
+    y, k = b.kv(u, v), b.assemble(u)[1]
+    out, k_out = torch.empty_like(y), torch.empty_like(k)
+
+    def sweeps():
+        a.kv(u, v, y_out=out, check_status=False)
+        a.assemble(u, want_f=False, k_out=k_out, check_status=False)
+
+    sweeps()
     g = torch.cuda.CUDAGraph()
     with torch.cuda.graph(g):
-        a.kv(u, v, y_out=out, check_status=False)
+        sweeps()
     out.zero_()
+    k_out.zero_()
     g.replay()
     torch.cuda.synchronize()
-    assert torch.equal(out, y)
+    assert torch.equal(out, y) and torch.equal(k_out, k)
