@@ -64,6 +64,10 @@ extern "C" {
  */
 size_t psx_status_bytes(void);
 
+/* Zero a status block on `stream`; copy it to host memory (best pinned) and wait for that. */
+int psx_status_reset(void* status, void* stream);
+int psx_status_read(const void* status, void* host, void* stream);
+
 /* ---- Sparsity pattern (host memory, once per mesh) ------------------------- */
 
 /*

@@ -52,6 +52,8 @@ SIGNATURES: dict[str, list] = {
     "psx_task_count": [_p, _i32, _i32, _i32, _i32, _p],
     "psx_task_fill": [_p, _i32, _i32, _i32, _i32, _p, _p],
     "psx_point_lists": [_p, _p],
+    "psx_status_reset": [_p, _p],
+    "psx_status_read": [_p, _p, _p],
     "psx_work_bytes": [_p, _i32, _p, _p],
     "psx_tet4_assemble": [_p, _p, _p, _p, _p, _f64, _f64, _f64, _i32, _i32, _p, _p, _p, _i64, _p, _p],
     "psx_tet4_kv": [_p, _p, _p, _p, _p, _f64, _f64, _i32, _p, _p, _p, _i64, _p, _p],
@@ -202,3 +204,33 @@ def ptr(t) -> int | None:
     if hasattr(t, "data_ptr"):
         return t.data_ptr()
     return t.ctypes.data
+
+
+def current_stream() -> int:
+    """Handle of the current stream of the current device."""
+    import torch
+
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+
+
+class DeviceStatus:
+    """A status block (``psx_status_bytes``) on the device, and pinned memory to read it through.
+
+    A checked f + K sweep of 3,840 elements took 52 us with a fill kernel and a pageable copy
+    through torch, 39 us with the memset and the pinned copy here (of which the read is 12).
+    """
+
+    def __init__(self, device):
+        import torch
+
+        n = (int(lib().psx_status_bytes()) + 3) // 4
+        self.words = torch.zeros(n, dtype=torch.int32, device=device)
+        self._host = torch.zeros(n, dtype=torch.int32, pin_memory=True)
+
+    def reset(self) -> None:
+        check(lib().psx_status_reset(self.words.data_ptr(), current_stream()), "psx_status_reset")
+
+    def read(self) -> list[int]:
+        """The words as of the work queued on the current stream (synchronises)."""
+        check(lib().psx_status_read(self.words.data_ptr(), self._host.data_ptr(), current_stream()), "psx_status_read")
+        return self._host.tolist()

@@ -28,10 +28,6 @@ from psierra_b200.pattern import MeshPattern
 PRECISIONS = {"fp64": _lib.PSX_FP64, "fp32-mixed": _lib.PSX_FP32_MIXED}
 
 
-def _stream_handle() -> int:
-    return torch.cuda.current_stream().cuda_stream
-
-
 WAIT_GAVE_UP = 1  # status flag bit 0: a bounded wait of a persistent kernel gave up
 
 
@@ -61,8 +57,8 @@ class GPUAssembler:
         self.precision = precision
         self.dev = self.pattern.device(self.device)
         self.X = torch.from_numpy(nodes).to(self.device)
-        nbytes = int(lib().psx_status_bytes())
-        self.status = torch.zeros((nbytes + 3) // 4, dtype=torch.int32, device=self.device)
+        self._status = _lib.DeviceStatus(self.device)
+        self.status = self._status.words
         self._dets = torch.zeros(8, dtype=torch.float64, device=self.device)
         self._work: dict = {}
         self.set_material(material)
@@ -166,7 +162,7 @@ class GPUAssembler:
             k_out = self.new_k(prec)
         if want_k and k_out.dtype != self.k_dtype(prec):
             raise ValueError(f"k_out must be {self.k_dtype(prec)} for precision {prec}")
-        self.status.zero_()
+        self._status.reset()
         work = self.workspace(prec)
         entry = lib().psx_tet4_assemble if self.npe == 4 else lib().psx_tet10_assemble
         rc = entry(
@@ -174,7 +170,7 @@ class GPUAssembler:
             ptr(self.mu_e), ptr(self.kappa_e), self.mu, self.kappa, self.rho if mass else self.lam, mode,
             PRECISIONS[prec],
             ptr(f_out) if want_f else None, ptr(k_out) if want_k else None, ptr(work), work.numel(),
-            ptr(self.status), _stream_handle())
+            ptr(self.status), _lib.current_stream())
         check(rc, "psx_tet4_assemble" if self.npe == 4 else "psx_tet10_assemble")
         if check_status:
             self.raise_on_bad_elements(u)
@@ -205,13 +201,13 @@ class GPUAssembler:
             k_out = self.new_k(prec)
         if k_out.dtype != self.k_dtype(prec):
             raise ValueError(f"k_out must be {self.k_dtype(prec)} for precision {prec}")
-        self.status.zero_()
+        self._status.reset()
         work = self.workspace(prec)
         mode = _lib.PSX_WANT_K | (_lib.PSX_WANT_F if want_f else 0)
         check(lib().psx_tet4_assemble_effective(
             ctypes.byref(self.dev["plan"]), ptr(self.X), ptr(u), ptr(self.mu_e), ptr(self.kappa_e), self.mu, self.kappa,
             self.lam, self.rho if rho is None else float(rho), float(c_t), float(c_m), float(c_0), mode, PRECISIONS[prec],
-            ptr(f_out) if want_f else None, ptr(k_out), ptr(work), work.numel(), ptr(self.status), _stream_handle()),
+            ptr(f_out) if want_f else None, ptr(k_out), ptr(work), work.numel(), ptr(self.status), _lib.current_stream()),
             "psx_tet4_assemble_effective")
         if check_status:
             self.raise_on_bad_elements(u)
@@ -251,11 +247,11 @@ class GPUAssembler:
         v = self._check_u(v)
         if y_out is None:
             y_out = self.new_f()
-        self.status.zero_()
+        self._status.reset()
         work = self.workspace(prec)
         check(lib().psx_tet4_kv(ctypes.byref(self.dev["plan"]), ptr(self.X), ptr(u), ptr(self.mu_e),
                                 ptr(self.kappa_e), self.mu, self.kappa, PRECISIONS[prec], ptr(v), ptr(y_out),
-                                ptr(work), work.numel(), ptr(self.status), _stream_handle()), "psx_tet4_kv")
+                                ptr(work), work.numel(), ptr(self.status), _lib.current_stream()), "psx_tet4_kv")
         if check_status:
             self.raise_on_bad_elements(u)
         return y_out
@@ -270,11 +266,11 @@ class GPUAssembler:
         gX = self.new_f()
         gmu = torch.empty(self.n_elements, dtype=torch.float64, device=self.device) if want_params else None
         gk = torch.empty(self.n_elements, dtype=torch.float64, device=self.device) if want_params else None
-        self.status.zero_()
+        self._status.reset()
         work = self.workspace("fp64")
         check(lib().psx_tet4_adjoint(ctypes.byref(self.dev["plan"]), ptr(self.X), ptr(u), ptr(self.mu_e),
                                      ptr(self.kappa_e), self.mu, self.kappa, ptr(w), ptr(gX), ptr(gmu), ptr(gk),
-                                     ptr(work), work.numel(), ptr(self.status), _stream_handle()),
+                                     ptr(work), work.numel(), ptr(self.status), _lib.current_stream()),
               "psx_tet4_adjoint")
         self.raise_on_bad_elements(u)
         return gX, gmu, gk
@@ -294,12 +290,12 @@ class GPUAssembler:
         u = self._check_u(u)
         for t in (b, minv, x, vel):
             self._check_u(t)
-        self.status.zero_()
+        self._status.reset()
         work = self.workspace(prec)
         check(lib().psx_tet4_dr_step(ctypes.byref(self.dev["plan"]), ptr(self.X), ptr(u), ptr(self.mu_e),
                                      ptr(self.kappa_e), self.mu, self.kappa, PRECISIONS[prec], ptr(b), ptr(minv),
                                      c1, c2, dt, ptr(x), ptr(vel), ptr(r_out), ptr(work), work.numel(),
-                                     ptr(self.status), _stream_handle()), "psx_tet4_dr_step")
+                                     ptr(self.status), _lib.current_stream()), "psx_tet4_dr_step")
         if check_status:
             self.raise_on_bad_elements(u)
 
@@ -313,9 +309,8 @@ class GPUAssembler:
     # ------------------------------------------------------------------ status
     def status_counts(self) -> tuple[int, int, int, int]:
         """(n_inverted, n_bad_volume, first_bad_element or -1, flags) of the last sweep (synchronises)."""
-        s = self.status[:6].cpu().numpy()
-        first = int(0x7FFFFFFF - int(s[2])) if s[2] != 0 else -1
-        return int(s[0]), int(s[1]), first, int(s[5])
+        s = self._status.read()
+        return s[0], s[1], 0x7FFFFFFF - s[2] if s[2] != 0 else -1, s[5]
 
     def last_spins(self) -> int:
         """Spin iterations the bounded waits of the last sweep took (synchronises)."""
@@ -329,7 +324,7 @@ class GPUAssembler:
         if self.npe == 10:
             # tet10_total_lagrangian.py:104-113: quadrature points in order, det J then det F
             check(lib().psx_tet10_element_dets(ptr(self.dev["conn"]), ptr(self.X), ptr(u), first,
-                                               ptr(self._dets), _stream_handle()), "psx_tet10_element_dets")
+                                               ptr(self._dets), _lib.current_stream()), "psx_tet10_element_dets")
             d = self._dets.cpu().numpy()
             for q in range(4):
                 if not d[2 * q] > 0.0:
@@ -338,7 +333,7 @@ class GPUAssembler:
                     raise ValueError(f"Element inversion detected: det(F) = {d[2 * q + 1]:.4e} <= 0.")
             raise ValueError("Element inversion detected: det(F) <= 0.")
         check(lib().psx_tet4_element_dets(ptr(self.dev["conn"]), ptr(self.X), ptr(u), first,
-                                          ptr(self._dets), _stream_handle()), "psx_tet4_element_dets")
+                                          ptr(self._dets), _lib.current_stream()), "psx_tet4_element_dets")
         detA, J = (float(v) for v in self._dets.cpu().numpy()[:2])
         if not detA > 0.0:
             raise ValueError(

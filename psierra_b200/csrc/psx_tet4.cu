@@ -1069,6 +1069,20 @@ int run_tet4_k32(const psx_plan_t* P, const Tet4Args& A, const WorkLayout& W, fl
 
 extern "C" size_t psx_status_bytes(void) { return sizeof(psx::Status); }
 
+extern "C" int psx_status_reset(void* status, void* stream) {
+  if (!status) return PSX_ERR_ARG;
+  return cudaMemsetAsync(status, 0, sizeof(psx::Status), static_cast<cudaStream_t>(stream)) == cudaSuccess
+             ? PSX_OK
+             : PSX_ERR_CUDA;
+}
+
+extern "C" int psx_status_read(const void* status, void* host, void* stream) {
+  if (!status || !host) return PSX_ERR_ARG;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (cudaMemcpyAsync(host, status, sizeof(psx::Status), cudaMemcpyDeviceToHost, s) != cudaSuccess) return PSX_ERR_CUDA;
+  return cudaStreamSynchronize(s) == cudaSuccess ? PSX_OK : PSX_ERR_CUDA;
+}
+
 extern "C" int psx_tet4_split_ready(void) {
   return psx::split_usable<float, PSX_WANT_F | PSX_WANT_K>() && psx::split_usable<float, PSX_WANT_K>() ? 1 : 0;
 }

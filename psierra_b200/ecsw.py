@@ -12,7 +12,7 @@ from __future__ import annotations
 import numpy as np
 import torch
 
-from psierra_b200._lib import check, lib, ptr
+from psierra_b200._lib import DeviceStatus, check, lib, ptr
 from psierra_b200.material import _host, material_moduli
 
 
@@ -44,19 +44,20 @@ class ECSWEvaluator:
         self.n = idx.size
         self.device = self.X.device
         self.work = torch.empty(int(lib().psx_ecsw_work_doubles(self.n, self.r)), dtype=torch.float64, device=dev)
-        self.status = torch.zeros((int(lib().psx_status_bytes()) + 3) // 4, dtype=torch.int32, device=dev)
+        self._status = DeviceStatus(dev)
+        self.status = self._status.words
 
     def evaluate_device(self, u_r: torch.Tensor):
         """``(f_r (r,), K_r (r, r))`` as device tensors for a device ``u_r``."""
         u_r = u_r.to(self.device, torch.float64).contiguous()
         f = torch.empty(self.r, dtype=torch.float64, device=self.device)
         K = torch.empty((self.r, self.r), dtype=torch.float64, device=self.device)
-        self.status.zero_()
+        self._status.reset()
         check(lib().psx_ecsw_evaluate(self.n, self.r, ptr(self.X), ptr(self.phi), ptr(self.w), ptr(u_r),
                                       ptr(self.mu_e), ptr(self.kappa_e), self.mu, self.kappa, ptr(f), ptr(K),
                                       ptr(self.work), self.work.numel(), ptr(self.status),
                                       torch.cuda.current_stream().cuda_stream), "psx_ecsw_evaluate")
-        s = self.status[:3].cpu().numpy()
+        s = self._status.read()
         if s[0] or s[1]:
             e = int(0x7FFFFFFF - int(s[2]))
             X = self.X[e].cpu().numpy().reshape(4, 3)

@@ -15,7 +15,7 @@ import numpy as np
 import scipy.sparse as spsp
 import torch
 
-from psierra_b200._lib import check, lib, ptr
+from psierra_b200._lib import DeviceStatus, check, lib, ptr
 from psierra_b200.material import material_moduli
 from psierra_b200.pattern import MeshPattern
 
@@ -72,8 +72,8 @@ class FbarAssembler:
         self.n_nbr = int(p.nbr_ptr[-1])
         nw = int(L.psx_fbar_work_doubles(self.n_elements, N, self.n_nbr))
         self.work = torch.empty(nw, dtype=torch.float64, device=self.device)
-        nbytes = int(L.psx_status_bytes())
-        self.status = torch.zeros((nbytes + 3) // 4, dtype=torch.int32, device=self.device)
+        self._status = DeviceStatus(self.device)
+        self.status = self._status.words
         self.jbar = torch.empty(self.n_elements, dtype=torch.float64, device=self.device)
 
     @property
@@ -90,7 +90,7 @@ class FbarAssembler:
             raise ValueError("u must be a float64 (3N,) tensor on the assembler's device")
         f = torch.empty(3 * self.n_nodes, dtype=torch.float64, device=self.device) if want_f else None
         k = torch.empty(self.nnz, dtype=torch.float64, device=self.device) if want_k else None
-        self.status.zero_()
+        self._status.reset()
         d = self.d
         check(lib().psx_fbar_assemble(
             ptr(d["conn"]), self.n_elements, self.n_nodes, ptr(d["X"]), ptr(u), self.mu, self.kappa, ptr(d["inc_ptr"]),
@@ -104,7 +104,7 @@ class FbarAssembler:
         return f, k
 
     def raise_on_bad_elements(self, u: torch.Tensor) -> None:
-        s = self.status[:4].cpu().numpy()
+        s = self._status.read()
         if s[0] == 0 and s[1] == 0:
             return
         e = int(0x7FFFFFFF - int(s[2]))
@@ -134,10 +134,10 @@ class FbarAssembler:
         n = jd.numel()
         k = torch.empty((n, 12, 12), dtype=torch.float64, device=self.device)
         f = torch.empty((n, 12), dtype=torch.float64, device=self.device)
-        self.status.zero_()
+        self._status.reset()
         check(lib().psx_fbar_element(n, ptr(Xd), ptr(ud), ptr(jd), self.mu, self.kappa, ptr(k), ptr(f),
                                      ptr(self.status), _stream()), "psx_fbar_element")
-        s = self.status[:4].cpu().numpy()
+        s = self._status.read()
         if s[0] or s[1]:
             e = int(0x7FFFFFFF - int(s[2]))
             X = np.asarray(X_elem, dtype=np.float64).reshape(-1, 4, 3)[e]

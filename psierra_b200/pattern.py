@@ -184,18 +184,16 @@ class MeshPattern:
         """The lists of the point records (``psx_point_lists``), on the device."""
         import torch
 
-        st, new = d["plan"], {}
+        st, new, h = d["plan"], {}, self.plan_host()
         for key in ("pair", "node"):
-            n = d[key + "_ptr"].numel() - 1
-            width = torch.zeros((n + 31) // 32 * 32, dtype=torch.int32, device=d["device"])
-            width[:n] = d[key + "_ptr"].diff()
-            ends = (width.view(-1, 32).amax(1).long() * 32).cumsum(0)
-            size = int(ends[-1]) if n else 0
-            if size > 4 * d[key + "_src"].numel() + 4096:  # a few long lists, mostly padding: the queue
+            width = np.diff(h[key + "_ptr"])
+            width = np.pad(width, (0, -width.size % 32)).reshape(-1, 32).max(axis=1, initial=0)
+            base = np.concatenate(([0], np.cumsum(32 * width, dtype=np.int64)))
+            size = int(base[-1])
+            if size > 4 * h[key + "_src"].size + 4096:  # a few long lists, mostly padding: the queue
                 return
-            base = torch.zeros(ends.numel() + 1, dtype=torch.int32, device=d["device"])
-            base[1:] = ends
-            new[key + "_base"], new[key + "_list"] = base, torch.empty(max(size, 1), dtype=torch.int32, device=d["device"])
+            new[key + "_base"] = torch_from(base.astype(np.int32), d["device"])
+            new[key + "_list"] = torch.empty(max(size, 1), dtype=torch.int32, device=d["device"])
         for k, v in new.items():
             setattr(st, k, v.data_ptr())
         stream = torch.cuda.current_stream()
