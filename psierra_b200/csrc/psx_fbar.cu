@@ -20,9 +20,9 @@
 // Kernels (one thread per element, node, one-ring entry or two-ring block; every sum in a
 // fixed order, the reference's ascending element / patch node but for the longest lists,
 // which a warp adds as a tree).  Measured on 162,000 elements, us (before): 11 (16), 9 (9),
-// 30 (51), 75 (122), 111 (154), 76 (96).  What bounds them: the volumetric pass its
-// instructions and gathered loads, the element pass 8 warps per SM at 248 registers, the
-// gather the latency of its records.
+// 30 (51), 54 (122), 111 (154), 59 (96).  What bounds them: the volumetric pass its
+// instructions and gathered loads, the element pass 12 warps per SM and its 134 MB of records,
+// the gather the latency of their loads.
 //   fbar_pre     V_e, J_e, q_e (and the inversion status)
 //   fbar_nodes   v0_a, J_node_a
 //   fbar_patch   g_a[b] = sum_{e in E_a, b in e} (V_e J_e / (4 v0_a)) q_e,b
@@ -41,10 +41,14 @@ namespace psx {
 namespace {
 
 constexpr int kFbThreads = 128;
-// Element record: 6 pair blocks (9 values in 10), 4 diagonal blocks (6), 4 forces (3 in 4),
-// each a whole number of 16-byte loads.  (Blocks padded for 32-byte loads made the records a
-// fifth larger: element pass 109 instead of 74 us on 162,000 elements, gather no faster.)
-constexpr int kFbPair = 10, kFbDiag = 6 * kFbPair, kFbForce = kFbDiag + 4 * 6, kFbRec = kFbForce + 4 * 4;
+// Element record, in planes over the elements: per pair block two quads and its ninth value,
+// per node f (a quad), the diagonal block's xx xy xz yy (a quad) and yz zz (a pair).  Whole
+// sectors for the stores of a warp, three loads per item; one 800-byte record per element,
+// staged through shared memory, took five (element pass 75 us, gather 76; now 54 and 59).
+constexpr int kFbRec = 96;  // doubles per element: 94 in whole 32-byte sectors
+__device__ __forceinline__ int64_t fb_quad(int64_t E, int i, int64_t e) { return (i * E + e) * 4; }
+__device__ __forceinline__ int64_t fb_ninth(int64_t E, int slot, int64_t e) { return (80 + slot) * E + e; }
+__device__ __forceinline__ int64_t fb_pair(int64_t E, int a, int64_t e) { return 86 * E + (a * E + e) * 2; }
 
 struct FbarArgs {
   const int32_t* conn;      // E x 4
@@ -109,9 +113,7 @@ __device__ __forceinline__ void fb_F(const double Un[4][3], const double g[4][3]
 }
 
 // Copy a block's records (n x len doubles, staged in shared memory with `stride` doubles per
-// record) to consecutive global memory, whole lines at a time.  A thread storing its own
-// record wrote eight bytes of 32 sectors per instruction: the element pass took 122 us on
-// 162,000 elements, now 75 (22.5M sector writes, now 6.1M).
+// record) to consecutive global memory, whole lines at a time.
 // `at(j)`: place of value j in the record of LEN doubles.
 template <int VALS, int STRIDE, int LEN, typename At>
 __device__ __forceinline__ void fb_copy_records(double* __restrict__ out, const double* s, int n, At at) {
@@ -242,11 +244,11 @@ __global__ void __launch_bounds__(kFbThreads) fbar_patch(FbarArgs A) {
   }
 }
 
-constexpr int kFbElemThreads = 64;  // 52 KB of staged records: four blocks per SM, as the registers allow
-constexpr int kFbRecStride = kFbRec + 1;
-__global__ void __launch_bounds__(kFbElemThreads, 4) fbar_element(FbarArgs A) {
-  extern __shared__ __align__(16) double s_rec[];
-  const int64_t e0 = blockIdx.x * (int64_t)kFbElemThreads, e = e0 + threadIdx.x;
+// Register target: 168, 12 warps per SM (148 bytes spilled).  F-bar sweep of 162,000 elements:
+// 312 us, with 209 registers and 8 warps 318.
+constexpr int kFbElemThreads = 64;
+__global__ void __launch_bounds__(kFbElemThreads, 6) fbar_element(FbarArgs A) {
+  const int64_t e = blockIdx.x * (int64_t)kFbElemThreads + threadIdx.x;
   if (e < A.E) {
     const int4 cn = reinterpret_cast<const int4*>(A.conn)[e];
     double Xn[4][3], Un[4][3], g[4][3], F[3][3], detD;
@@ -301,6 +303,31 @@ __global__ void __launch_bounds__(kFbElemThreads, 4) fbar_element(FbarArgs A) {
         Sb[j][i] = m;
       }
     const double trS = Sb[0][0] + Sb[1][1] + Sb[2][2];
+    // g_b^T S_bar g_c of the ten blocks, and f: g, S_bar and F are not needed after them
+    // f_b = V F [r^2 S_bar + (1 - r^2) tr(S_bar)/3 I] g_b
+    double gsg[10];
+#pragma unroll
+    for (int a = 0, at = 0; a < 4; ++a)
+#pragma unroll
+      for (int b = a; b < 4; ++b, ++at) {
+        gsg[at] = 0.0;
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+#pragma unroll
+          for (int j = 0; j < 3; ++j) gsg[at] += g[a][i] * Sb[i][j] * g[b][j];
+      }
+    const double r2 = r * r;
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+      double w[3], f[3];
+#pragma unroll
+      for (int i = 0; i < 3; ++i)
+        w[i] = r2 * (Sb[i][0] * g[b][0] + Sb[i][1] * g[b][1] + Sb[i][2] * g[b][2]) +
+               (1.0 - r2) * (trS / 3.0) * g[b][i];
+#pragma unroll
+      for (int k = 0; k < 3; ++k) f[k] = V * (F[k][0] * w[0] + F[k][1] * w[1] + F[k][2] * w[2]);
+      st_quad(A.rec + fb_quad(A.E, 12 + b, e), Quad{f[0], f[1], f[2], 0.0});
+    }
     // per node: p = F^-T g, q = F g, t = (F F^T)^-1 p = F^-T F^-1 p, s = p - tr(C^-1)/3 q
     double p[4][3], qv[4][3], t[4][3], s[4][3];
     double Ci[3][3];  // C^-1 = F^-1 F^-T
@@ -332,20 +359,15 @@ __global__ void __launch_bounds__(kFbElemThreads, 4) fbar_element(FbarArgs A) {
     }
     const double Ap = A.kappa + (2.0 / 9.0) * phib * I1b;
     const double Bp = (2.0 / 3.0) * phib * I1b - 2.0 * A.kappa * lnJb;
-    double* R = s_rec + kFbRecStride * threadIdx.x;
     const int gid[4] = {cn.x, cn.y, cn.z, cn.w};
     int slot = 0;
 #pragma unroll
-    for (int a = 0; a < 4; ++a)
+    for (int a = 0, at = 0; a < 4; ++a)
 #pragma unroll
-      for (int b = a; b < 4; ++b) {
-        double gsg = 0.0, pp = 0.0;
+      for (int b = a; b < 4; ++b, ++at) {
+        double pp = 0.0;
 #pragma unroll
-        for (int i = 0; i < 3; ++i) {
-          pp += p[a][i] * p[b][i];
-#pragma unroll
-          for (int j = 0; j < 3; ++j) gsg += g[a][i] * Sb[i][j] * g[b][j];
-        }
+        for (int i = 0; i < 3; ++i) pp += p[a][i] * p[b][i];
         double v[3][3];
 #pragma unroll
         for (int k = 0; k < 3; ++k)
@@ -354,38 +376,26 @@ __global__ void __launch_bounds__(kFbElemThreads, 4) fbar_element(FbarArgs A) {
             double x = Ap * s[a][k] * s[b][m] +
                        Bp * (0.5 * p[b][k] * p[a][m] - (t[a][k] * qv[b][m] + qv[a][k] * t[b][m]) / 3.0 +
                              (trCi2 / 9.0) * qv[a][k] * qv[b][m]);
-            if (k == m) x += Bp * 0.5 * pp + gsg;
+            if (k == m) x += Bp * 0.5 * pp + gsg[at];
             v[k][m] = V * x;
           }
         if (a == b) {
-          double* d = R + kFbDiag + 6 * a;
-          d[0] = v[0][0]; d[1] = v[0][1]; d[2] = v[0][2]; d[3] = v[1][1]; d[4] = v[1][2]; d[5] = v[2][2];
+          st_quad(A.rec + fb_quad(A.E, 16 + a, e), Quad{v[0][0], v[0][1], v[0][2], v[1][1]});
+          *reinterpret_cast<double2*>(A.rec + fb_pair(A.E, a, e)) = make_double2(v[1][2], v[2][2]);
         } else {
-          double* o = R + kFbPair * slot;
           const bool swap = gid[a] > gid[b];  // rows = the node of smaller global id
+          double o[9];
 #pragma unroll
           for (int k = 0; k < 3; ++k)
 #pragma unroll
             for (int m = 0; m < 3; ++m) o[3 * k + m] = swap ? v[m][k] : v[k][m];
+          st_quad(A.rec + fb_quad(A.E, 2 * slot, e), Quad{o[0], o[1], o[2], o[3]});
+          st_quad(A.rec + fb_quad(A.E, 2 * slot + 1, e), Quad{o[4], o[5], o[6], o[7]});
+          A.rec[fb_ninth(A.E, slot, e)] = o[8];
           ++slot;
         }
       }
-    // f_b = V F [r^2 S_bar + (1 - r^2) tr(S_bar)/3 I] g_b
-    const double r2 = r * r;
-#pragma unroll
-    for (int b = 0; b < 4; ++b) {
-      double w[3];
-#pragma unroll
-      for (int i = 0; i < 3; ++i)
-        w[i] = r2 * (Sb[i][0] * g[b][0] + Sb[i][1] * g[b][1] + Sb[i][2] * g[b][2]) +
-               (1.0 - r2) * (trS / 3.0) * g[b][i];
-#pragma unroll
-      for (int k = 0; k < 3; ++k) R[kFbForce + 4 * b + k] = V * (F[k][0] * w[0] + F[k][1] * w[1] + F[k][2] * w[2]);
-    }
   }
-  __syncthreads();
-  fb_copy_records<kFbRec, kFbRecStride, kFbRec>(A.rec + (int64_t)kFbRec * e0, s_rec,
-                                                (int)min((int64_t)kFbElemThreads, A.E - e0), [](int j) { return j; });
 }
 
 struct FbarGather {
@@ -395,7 +405,7 @@ struct FbarGather {
   const int32_t* node_info2;
   const int32_t* node_ptr;
   const int32_t* node_src;    // e * 16 + local node
-  int64_t n_pairs, n_nodes;
+  int64_t n_pairs, n_nodes, E;
 };
 
 __device__ __forceinline__ int4 fb_info(const int32_t* p) { return make_int4(__ldg(p), __ldg(p + 1), __ldg(p + 2), __ldg(p + 3)); }
@@ -420,14 +430,12 @@ __global__ void __launch_bounds__(kFbThreads) fbar_gather(FbarGather G, const do
         for (int b = 0; b < kFbBatch; ++b)
           if (s + b < s1) {
             const int32_t c = __ldg(G.pair_src + s + b);
-            const double2* o = reinterpret_cast<const double2*>(rec + (int64_t)kFbRec * (c >> 6) + kFbPair * (c & 63));
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              const double2 x = __ldg(o + j);
-              v[b][2 * j] = x.x;
-              v[b][2 * j + 1] = x.y;
-            }
-            v[b][8] = __ldg(reinterpret_cast<const double*>(o + 4));
+            const int slot = c & 63;
+            const int64_t e = c >> 6;
+            const Quad x = ld_quad_nc(rec + fb_quad(G.E, 2 * slot, e)), y = ld_quad_nc(rec + fb_quad(G.E, 2 * slot + 1, e));
+            v[b][0] = x.x; v[b][1] = x.y; v[b][2] = x.z; v[b][3] = x.w;
+            v[b][4] = y.x; v[b][5] = y.y; v[b][6] = y.z; v[b][7] = y.w;
+            v[b][8] = __ldg(rec + fb_ninth(G.E, slot, e));
           }
 #pragma unroll
         for (int b = 0; b < kFbBatch; ++b)
@@ -451,18 +459,13 @@ __global__ void __launch_bounds__(kFbThreads) fbar_gather(FbarGather G, const do
         for (int b = 0; b < kFbBatch; ++b)
           if (s + b < s1) {
             const int32_t c = __ldg(G.node_src + s + b);
-            const double2* R = reinterpret_cast<const double2*>(rec + (int64_t)kFbRec * (c >> 4));
             const int a = c & 15;
-#pragma unroll
-            for (int j = 0; j < 3; ++j) {
-              const double2 x = __ldg(R + kFbDiag / 2 + 3 * a + j);
-              v[b][2 * j] = x.x;
-              v[b][2 * j + 1] = x.y;
-            }
-            const double2 y = __ldg(R + kFbForce / 2 + 2 * a);
-            v[b][6] = y.x;
-            v[b][7] = y.y;
-            v[b][8] = __ldg(reinterpret_cast<const double*>(R + kFbForce / 2 + 2 * a + 1));
+            const int64_t e = c >> 4;
+            const Quad x = ld_quad_nc(rec + fb_quad(G.E, 12 + a, e)), y = ld_quad_nc(rec + fb_quad(G.E, 16 + a, e));
+            const double2 z = __ldg(reinterpret_cast<const double2*>(rec + fb_pair(G.E, a, e)));
+            v[b][0] = y.x; v[b][1] = y.y; v[b][2] = y.z; v[b][3] = y.w;
+            v[b][4] = z.x; v[b][5] = z.y;
+            v[b][6] = x.x; v[b][7] = x.y; v[b][8] = x.z;
           }
 #pragma unroll
         for (int b = 0; b < kFbBatch; ++b)
@@ -697,12 +700,9 @@ extern "C" int psx_fbar_assemble(const int32_t* conn, int64_t E, int64_t N, cons
   // two-ring CSR holds 9 values per entry
   if (k_out)
     fbar_vol<<<fb_grid(nnz2 / 9), kFbThreads, 0, s>>>(N, nbr2_ptr, vol_ptr, vol_src, A.g, k_out);
-  constexpr int kElemSmem = sizeof(double) * kFbElemThreads * kFbRecStride;
-  static unsigned long long s_smem_set = 0;
-  if (set_dynamic_smem_once(fbar_element, kElemSmem, &s_smem_set) != cudaSuccess) return PSX_ERR_CUDA;
   if ((E + kFbElemThreads - 1) / kFbElemThreads > 0x7fffffff) return PSX_ERR_LIMIT;
-  fbar_element<<<(unsigned)((E + kFbElemThreads - 1) / kFbElemThreads), kFbElemThreads, kElemSmem, s>>>(A);
-  FbarGather G{pair_info2, pair_ptr, pair_src, node_info2, node_ptr, node_src, n_pairs, N};
+  fbar_element<<<(unsigned)((E + kFbElemThreads - 1) / kFbElemThreads), kFbElemThreads, 0, s>>>(A);
+  FbarGather G{pair_info2, pair_ptr, pair_src, node_info2, node_ptr, node_src, n_pairs, N, E};
   fbar_gather<<<fb_grid(n_pairs + N), kFbThreads, 0, s>>>(G, A.rec, k_out, f_out);
   PSX_CUDA_CHECK_LAUNCH();
   return PSX_OK;
