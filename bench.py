@@ -39,11 +39,11 @@ def workload(cells: int, elements: int, nodes: int) -> str:
             "u=0.05 sin(pi x) sin(pi y) z e_z + U(+-1e-4); one fused f_int+K_T assembly per step")
 
 
-# DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of one launch, from one ncu
-# capture of the FP32-mixed f+K and K.v launches on the cube 56^3 (1,053,696 elements);
+# DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of one sweep's two launches, from
+# an ncu capture of the FP32-mixed f+K and K.v sweeps on the cube 56^3 (1,053,696 elements);
 # the traffic grows with the element count, so it is scaled by E for this workload.
 NCU_CAPTURE_ELEMENTS = 1053696
-NCU_TRAFFIC = {"fk32": 98.47552e6 + 102.580736e6, "kv32": 52.138752e6 + 1.884416e6}
+NCU_TRAFFIC = {"fk32": 292.361216e6 + 174.428928e6, "kv32": 87.758336e6 + 2.580736e6}
 
 
 def parse():
@@ -296,10 +296,10 @@ def dr_benchmark(asm, k_vals, u_dev, m, iterations: int, sync_all, cells: int = 
 
 
 # FP64 floating-point work of the FP64 f+K element sweep, per element: 2 x DFMA + DADD + DMUL
-# thread instructions of tet4_persistent_kernel<double, F|K> from the ncu counters
-# smsp__sass_thread_inst_executed_op_d{fma,add,mul}_pred_on.sum of one launch on the 56^3
-# cube (467.8M, 207.6M, 250.8M for 1,053,696 elements).
-FP64_FLOPS_PER_ELEMENT = (2 * 467841024 + 207578112 + 250779648) / 1053696
+# thread instructions of tet4_points_kernel and tet4_point_items_kernel<double, F|K> from the
+# ncu counters smsp__sass_thread_inst_executed_op_d{fma,add,mul}_pred_on.sum of one sweep of
+# the 56^3 cube (460.5M, 147.5M, 264.5M for 1,053,696 elements).
+FP64_FLOPS_PER_ELEMENT = (2 * 460465152 + 147517440 + 264477696) / 1053696
 
 
 def fp64_compute_roofline(E, ms, roofs):
@@ -629,7 +629,9 @@ def main():
         from psierra_b200 import _lib
 
         split = asm.pattern.split and _lib.lib().psx_tet4_split_ready() == 1
-        fk_kernel = ("tet4_split_kernel<float> F|K (per SM 8 element-tile warps + 8 owner-computes gather warps, "
+        fk_kernel = ("tet4_points_kernel<float> F|K (element factors), then tet4_point_items_kernel<float> (blocks "
+                     "formed and summed, one thread per node pair and node)" if asm.dev["plan"].two_pass_p & 2 else
+                     "tet4_split_kernel<float> F|K (per SM 8 element-tile warps + 8 owner-computes gather warps, "
                      "registers moved between them by setmaxnreg)" if split else
                      "tet4_persistent_kernel<float> F|K (element tiles + owner-computes gather in the same warps)")
         line = {
@@ -644,8 +646,8 @@ def main():
                        "parallelism": f"replicas x{world}" if world > 1 else "single GPU"},
             "roofline": {"bound": "hbm", "achieved": ach, "peak": peak, "unit": "GB/s", "frac": ach / peak,
                          "traffic": NCU_TRAFFIC["fk32"] * E / NCU_CAPTURE_ELEMENTS,
-                         "traffic_note": "bytes per launch: ncu DRAM read+write of the cube 56^3 launch scaled by "
-                                         "elements (latency-bound: DRAM throughput 10.7% in that capture of the split kernel)",
+                         "traffic_note": "bytes per sweep: ncu DRAM read+write of the cube 56^3 sweep's two launches scaled by "
+                                         "elements (latency-bound: DRAM throughput 30% and 34% in that capture)",
                          "peak_kind": peak_kind,
                          "algorithmic_bytes_per_launch": bytes_mixed, "kernel": fk_kernel,
                          "launches_per_step": asm.launches_per_call("fp32-mixed")},
@@ -670,7 +672,7 @@ def main():
             "pcg": pcg,
             "dynamic_relaxation": dr,
             "cpu_baseline": cb, "e2e": e2e, "gpu_launches": args.steps * asm.launches_per_call("fp32-mixed"),
-            "gpu_launches_note": "assembly timed region; each K.v step is one launch as well",
+            "gpu_launches_note": "assembly timed region; each K.v step is two launches",
             "clocks": clk,
         }
         print(json.dumps(line))

@@ -279,10 +279,11 @@ int psx_work_bytes(const psx_plan_t* plan, int precision, int64_t* ring_elems, i
  *   f_out (device, 3N doubles) when mode has PSX_WANT_F
  *   k_out (device, nnz values in psx_csr_pattern order: double for PSX_FP64, float
  *          for PSX_FP32_MIXED) when mode has PSX_WANT_K or PSX_LINEAR
- *   work (device, >= psx_work_bytes, 256-byte aligned) scratch ring of element records
+ *   work (device, >= psx_work_bytes, 256-byte aligned) scratch: records of the elements
  *   status (device, psx_status_bytes(), zeroed by the caller); flags bit 0 is set if a
  *          bounded wait of the persistent kernel gave up (the results are then invalid)
- * One launch of a persistent kernel; the call also clears the task counters.
+ * Two launches where the plan says so (two_pass, two_pass_k, two_pass_p), else one of a
+ * persistent kernel, and the task counters cleared.
  * Deterministic: every output value is a fixed-order sum; no atomics touch f or K.
  */
 int psx_tet4_assemble(const psx_plan_t* plan, const double* X, const double* u,
@@ -427,7 +428,9 @@ int psx_pcg_work_bytes(int64_t n, int precond, int64_t* bytes);
  * after maxiter updates without that it stops unconverged.  Writes to status:
  * iters = iterations, flags = 0 converged / 2 max iterations reached / 4 breakdown,
  * value = final ||r||.  Dot products are reduced in a fixed order (bitwise
- * reproducible).  Synchronises the stream every 16 iterations to test convergence.
+ * reproducible).  A system whose state fits the GPU's shared memory (176 bytes per node with
+ * block-Jacobi and nodal rows: about 578,000 unknowns) is solved in one launch, without host
+ * reads; above that the call synchronises the stream every 16 iterations to test convergence.
  */
 int psx_pcg(int64_t n, const int32_t* indptr, const int32_t* indices, const void* values,
             int value_precision, const double* b, double* x, double rtol, double atol, int32_t maxiter,
@@ -552,8 +555,9 @@ int psx_csr_dirichlet(int64_t n, const int32_t* indptr, const int32_t* indices, 
  * before its run either sets CUDA_MODULE_LOADING=EAGER or makes one psx_pcg_static call
  * on each device during its set-up; later calls reserve nothing more.  The first call on
  * a device also looks up the scratch address on that device; make that first call before
- * any stream capture.  Like psx_pcg, the solve reads its convergence test back to the
- * host every 16 iterations (a device-to-host copy and a synchronisation of `stream`).
+ * any stream capture.  Like psx_pcg, a system that one launch does not take has its
+ * convergence test read back to the host every 16 iterations (a device-to-host copy and a
+ * synchronisation of `stream`).
  * Every call on a device shares the one array, so calls that overlap on the GPU (other
  * streams, other host threads) race; the scalars the solve needs at zero are cleared at
  * the start of every call.  Arguments and results are those of psx_pcg.

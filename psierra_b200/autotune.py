@@ -11,6 +11,10 @@ in separate warps (the warp-specialised kernel, whose ring is sized by the same 
 slack) or in the same ones.  ``tune`` times each candidate with CUDA events on the
 caller's stream and keeps the fastest; results are cached per device, element type,
 mesh size and precision, in memory and optionally in a JSON file.
+
+Sweeps that also run in two launches without a queue are timed that way last, and keep it when
+it is faster.  That changes no bit either, but for the FP32 tangents of meshes large enough for
+point records (``MeshPattern.POINT_ELEMENTS_FP32``), whose sums are associated differently.
 """
 from __future__ import annotations
 

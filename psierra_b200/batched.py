@@ -3,8 +3,8 @@
 pSierra solves one mesh per ``NonlinearStaticAnalysis`` (psierra
 ``analysis/nonlinear_static.py:250-404``); a study over many specimens loops over
 them in Python.  Here a batch of Tet4 meshes becomes the disjoint union of their
-meshes (``meshgen.concat_meshes``) with per-element moduli, so one persistent
-``psx_tet4_assemble`` launch evaluates every element of every instance, whatever the
+meshes (``meshgen.concat_meshes``) with per-element moduli, so one
+``psx_tet4_assemble`` call evaluates every element of every instance, whatever the
 instance sizes, and the union's CSR pattern is block diagonal by construction.
 
 ``BatchedNewton`` runs the incremental Newton of every instance at once.  One Newton

@@ -5,17 +5,18 @@
 // (element/tet4_total_lagrangian.py:77-139) and the COO->CSR / np.add.at scatter
 // (utility/assembly.py:37-108).
 //
-// Two phases per element chunk, fused into one launch per chunk:
-//   A (element-centric): one thread per element evaluates the kinematics, the NeoHookean
-//     stress and tangent, its 10 distinct 3x3 tangent blocks and its 4 nodal force
-//     vectors, once, and writes them to an L2-resident ring of element records
-//     (psx_gather.cuh).
+// Two phases:
+//   A (element-centric): one thread per element evaluates the kinematics and the NeoHookean
+//     stress and tangent once and writes a record (psx_gather.cuh): its factors (point records),
+//     its blocks and forces (element records), or its warp's summed ones (tile records).
 //   B (owner-computes gather): one thread per node pair / node sums the records of the
 //     elements that share it, in ascending element order, and writes each CSR value and
 //     each f entry exactly once.
-// Both phases run in one persistent launch that drains a task queue in mesh order, so
-// the ring only holds the elements still awaited by some gather item.  No atomics touch f or K, so
-// results are bitwise reproducible run to run.
+// The phases are two launches on records of the whole mesh (tet4_points_kernel,
+// tet4_tiles_kernel), or one persistent launch that drains a task queue in mesh order over
+// an L2-resident ring, which holds only the elements still awaited by some gather item (meshes
+// whose records would grow too large).  No atomics touch f or K, so results are bitwise
+// reproducible run to run.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -580,12 +581,12 @@ tet4_split_kernel(Tet4Args A, GatherArgs g, QueueArgs Q, const int4* __restrict_
 // association as the queue, so the same bits; but no claims, waits or completion counts, warps
 // that hold only what an element tile needs, and gathers at full occupancy instead of a turn
 // in the queue.  The records of the whole mesh are kept (22 bytes per element without a
-// tangent, in L2 up to about 5M elements; 141 with one, so larger meshes queue:
-// psierra_b200/pattern.py has the line).  Measured, queue -> two passes, us:
+// tangent, in L2 up to about 5M elements; 141 with one: psierra_b200/pattern.py has the
+// lines).  Measured, queue -> two passes, us:
 //   elements    f              K.v FP32        K.v FP64      f + K FP32
 //     384,000    71 ->  25      69 ->  31       80 ->  33     119 ->  91
-//   1,053,696   106 ->  56     120 ->  68      121 ->  80     237 -> 244 (queued)
-//   3,072,000   272 -> 146     297 -> 181      320 -> 220     639 -> 672 (queued)
+//   1,053,696   106 ->  56     120 ->  68      121 ->  80     237 -> 244 (point records)
+//   3,072,000   272 -> 146     297 -> 181      320 -> 220     639 -> 672 (point records)
 // What bounds them now: without a tangent the latency of the FP64 element chain (the FP64
 // pipe alone would take 21 us at 1.05M elements); with one, half each, pass 1 at 12 warps per
 // SM (shared memory of the staged blocks) and the scattered record reads and 12-byte row

@@ -245,12 +245,13 @@ class MeshPattern:
         their queue is chosen (``set_queue(lag_f=...)``) or its waits are limited."""
         return not self.queued_f and self.wait_spins == 0
 
-    # Elements up to which tangent sweeps run in two passes too.  Tet4, FP32: their records (141
-    # bytes per element) then stay in L2 between the passes; f + K on Kuhn cubes, us, two
-    # passes / queue: 82,944 elements 27 / 42, 196,608 47 / 85, 384,000 91 / 119, 663,552
-    # 159 / 209, 1,053,696 234 / 235, 3,072,000 652 / 630.  Tet10: two passes stay ahead (750,000
-    # elements, FP64, 3280 / 4000 us), but their records (5.2 KB per element) grow with the
-    # mesh, here to 4.1 GB; the queue's ring does not.
+    # Elements up to which tangent sweeps run in two passes too.  Tet4, FP32 (above
+    # POINT_ELEMENTS_FP32 the effective tangent alone): their records (141 bytes per element) then
+    # stay in L2 between the passes; f + K on Kuhn cubes, us, two passes / queue: 82,944 elements
+    # 27 / 42, 196,608 47 / 85, 384,000 91 / 119, 663,552 159 / 209, 1,053,696 234 / 235,
+    # 3,072,000 652 / 630.  Tet10: two passes stay ahead (750,000 elements, FP64, 3280 / 4000
+    # us), but their records (5.2 KB per element) grow with the mesh, here to 4.1 GB; the
+    # queue's ring does not.
     TWO_PASS_K_ELEMENTS = 3 << 18
 
     @property

@@ -90,3 +90,32 @@ def test_status_of_zero_load_limits_and_starts(n):
     z[7] = np.nan
     _, r = _solve(A, z, "block-jacobi", True)
     assert not r.converged
+
+
+@pytest.mark.parametrize("n", [300, 30000])
+def test_enqueued_in_a_graph(n):
+    from psierra_b200 import _lib
+
+    A, b = _system(n, True, seed=2)
+    want, r = _solve(A, b, "block-jacobi", True)
+    t = lambda a, d: torch.from_numpy(np.ascontiguousarray(a, dtype=d)).to(DEV)  # noqa: E731
+    ip, ix, v, bd = t(A.indptr, np.int32), t(A.indices, np.int32), t(A.data, np.float64), t(b, np.float64)
+    x, st = torch.zeros(n, dtype=torch.float64, device=DEV), torch.zeros(8, dtype=torch.int32, device=DEV)
+    precond = _lib.PSX_PRECOND_BJACOBI | _lib.PSX_PCG_NODAL
+    work = ConjugateGradientSolver(preconditioner="block-jacobi")._workspace(n, precond)
+
+    def solve():
+        x.zero_()
+        _lib.check(_lib.lib().psx_pcg_enqueue(n, ip.data_ptr(), ix.data_ptr(), v.data_ptr(), _lib.PSX_FP64, bd.data_ptr(),
+                                              x.data_ptr(), 1e-10, 0.0, 500, precond, work.data_ptr(), work.numel(),
+                                              st.data_ptr(), _lib.current_stream()), "psx_pcg_enqueue")
+
+    solve()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        solve()
+    for _ in range(2):
+        x.fill_(7.0)
+        g.replay()
+        torch.cuda.synchronize()
+        assert np.array_equal(x.cpu().numpy(), want) and int(st[4]) == r.iterations and int(st[5]) == 0
