@@ -191,7 +191,8 @@ typedef struct psx_plan {
  * of the 32 lists. */
 int psx_point_lists(const psx_plan_t* plan, void* stream);
 
-/* n_pairs = (sum deg - N) / 2 and the pair_src length E * npe (npe - 1) / 2 (host). */
+/* n_pairs = (sum deg - nodes of any element) / 2 and the pair_src length E * npe (npe - 1) / 2
+ * (host). */
 int psx_plan_count(const int64_t* conn, int64_t E, int npe, int64_t N, const int32_t* nbr_ptr,
                    int64_t* n_pairs, int64_t* n_pair_src);
 

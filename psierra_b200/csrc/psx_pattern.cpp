@@ -174,6 +174,14 @@ inline int local_pair_index(int a, int b, int npe) {  // a < b
   return a * npe - a * (a + 1) / 2 + (b - a - 1);
 }
 
+// Edges of the node graph.  A node of an element is in its own list, a node of none has an
+// empty one.
+int64_t count_pairs(const int32_t* nbr_ptr, int64_t N) {
+  int64_t used = 0;
+  for (int64_t i = 0; i < N; ++i) used += nbr_ptr[i + 1] > nbr_ptr[i];
+  return ((int64_t)nbr_ptr[N] - used) / 2;
+}
+
 struct Item {
   int32_t ready;
   int32_t order;  // tie break: original item index
@@ -185,7 +193,7 @@ extern "C" int psx_plan_count(const int64_t* conn, int64_t E, int npe, int64_t N
                               int64_t* n_pairs, int64_t* n_pair_src) {
   if (!args_ok(conn, E, npe, N) || !nbr_ptr || !n_pairs || !n_pair_src) return PSX_ERR_ARG;
   if (E > ((int64_t)1 << 25)) return PSX_ERR_LIMIT;  // slot encoding e * 64 + slot must fit int32
-  *n_pairs = ((int64_t)nbr_ptr[N] - N) / 2;
+  *n_pairs = count_pairs(nbr_ptr, N);
   *n_pair_src = E * (int64_t)(npe * (npe - 1) / 2);
   return PSX_OK;
 }
@@ -201,7 +209,7 @@ extern "C" int psx_plan_fill(const int64_t* conn, int64_t E, int npe, int64_t N,
   std::vector<int32_t> ptr, elem;
   std::vector<int8_t> local;
   incidences(conn, E, npe, N, ptr, elem, local);
-  const int64_t n_pairs = ((int64_t)nbr_ptr[N] - N) / 2;
+  const int64_t n_pairs = count_pairs(nbr_ptr, N);
   const int64_t n_gran = (E + granule - 1) / granule;
 
   // ---- pairs in (i, j) order: contributions = inc(i) intersect inc(j)
@@ -216,6 +224,7 @@ extern "C" int psx_plan_fill(const int64_t* conn, int64_t E, int npe, int64_t N,
     for (int32_t r = 0; r < deg; ++r) {
       const int64_t j = nbr[b0 + r];
       if (j <= i) continue;
+      if (p == n_pairs) return PSX_ERR_ARG;
       const int32_t* ej = nbr + nbr_ptr[j];
       const int32_t degj = nbr_ptr[j + 1] - nbr_ptr[j];
       const int32_t rji = (int32_t)(std::lower_bound(ej, ej + degj, (int32_t)i) - ej);
