@@ -61,6 +61,7 @@ class GPUAssembler:
         self.status = self._status.words
         self._dets = torch.zeros(8, dtype=torch.float64, device=self.device)
         self._work: dict = {}
+        self._work_layout = None
         self.set_material(material)
 
     # ------------------------------------------------------------------ material
@@ -103,25 +104,25 @@ class GPUAssembler:
 
     def set_queue(self, lag: int | None = None, blocks_per_sm: int | None = None,
                   ring_slack: int | None = None, lag_f: int | None = None, split: bool | None = None) -> None:
-        """Launch shape of the persistent kernel (see ``MeshPattern.set_queue``)."""
-        p = self.pattern
-        old = (p.lag, p.lag_f, p.ring_slack, p.two_pass, p.two_pass_k, p.point_precisions)
-        p.set_queue(lag=lag, blocks_per_sm=blocks_per_sm, ring_slack=ring_slack, lag_f=lag_f, split=split)
-        if (p.lag, p.lag_f, p.ring_slack, p.two_pass, p.two_pass_k, p.point_precisions) != old:
-            self._work.clear()  # the records are sized by the lag, the slack and the passes
+        """Launch shape of the persistent kernel (see ``MeshPattern.set_queue``), for every
+        assembler of this pattern.  Sweeps captured in a graph before are captured again."""
+        self.pattern.set_queue(lag=lag, blocks_per_sm=blocks_per_sm, ring_slack=ring_slack, lag_f=lag_f, split=split)
 
     def set_two_pass(self, f: bool = True, k: bool = True) -> None:
         """Back to the two-pass sweeps after ``set_queue`` (see ``MeshPattern.two_pass``)."""
         self.pattern.set_two_pass(f, k)
-        self._work.clear()
 
     def set_wait_limit(self, spins: int) -> None:
         """Polls after which a bounded wait of the persistent kernels gives up (0 = the
         default, about a second); see ``MeshPattern.set_wait_limit``."""
         self.pattern.set_wait_limit(spins)
-        self._work.clear()  # a limit selects the queued kernels, whose records are a ring
 
     def workspace(self, precision: str) -> torch.Tensor:
+        layout = self.dev["layout"]
+        if layout != self._work_layout:
+            # the pattern's queue or passes were chosen anew, by this assembler or another one
+            self._work.clear()
+            self._work_layout = layout
         w = self._work.get(precision)
         if w is None:
             ring = ctypes.c_int64()

@@ -238,6 +238,9 @@ class MeshPattern:
         st.two_pass_p = self.point_precisions if "pair_list" in d else 0
         st.n_gtasks_k = d["n_gtasks_k"] if on else 0
         st.gtasks_k = d["gtasks_k"].data_ptr() if on else None
+        # what psx_work_bytes depends on: every assembler of this pattern compares it with the
+        # one its workspace was made for
+        d["layout"] = (self.lag, self.lag_f, self.ring_slack, st.two_pass, st.two_pass_k, st.two_pass_p)
 
     @property
     def two_pass(self) -> bool:
