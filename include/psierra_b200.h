@@ -427,7 +427,8 @@ int psx_pcg_work_bytes(int64_t n, int precond, int64_t* bytes);
  * device; b (n) and x (n, in: initial guess -- zero for the reference's behaviour --,
  * out: solution) double.  Stops when ||r|| < max(atol, rtol ||b||), as scipy does;
  * after maxiter updates without that it stops unconverged.  Writes to status:
- * iters = iterations, flags = 0 converged / 2 max iterations reached / 4 breakdown,
+ * iters = iterations, flags = 0 converged / 2 max iterations reached / 4 breakdown / 1 a
+ * bounded wait of the one-launch form gave up (x is then invalid),
  * value = final ||r||.  Dot products are reduced in a fixed order (bitwise
  * reproducible).  A system whose state fits the GPU's shared memory (176 bytes per node with
  * block-Jacobi and nodal rows: about 578,000 unknowns) is solved in one launch, without host
@@ -446,6 +447,17 @@ int psx_pcg(int64_t n, const int32_t* indptr, const int32_t* indices, const void
 int psx_pcg_enqueue(int64_t n, const int32_t* indptr, const int32_t* indices, const void* values,
                     int value_precision, const double* b, double* x, double rtol, double atol, int32_t maxiter,
                     int precond, void* work, int64_t work_bytes, void* status, void* stream);
+
+/*
+ * psx_pcg (host_checks = 1) or psx_pcg_enqueue (0) with a limit on the waits of the one-launch
+ * form: its blocks meet three times per iteration, and after wait_spins polls of one meeting
+ * (0 = the default, 1 << 21, a second or two) a block gives up, the launch ends and status flag
+ * bit 0 is set.
+ */
+int psx_pcg_limited(int64_t n, const int32_t* indptr, const int32_t* indices, const void* values,
+                    int value_precision, const double* b, double* x, double rtol, double atol, int32_t maxiter,
+                    int precond, void* work, int64_t work_bytes, void* status, void* stream, int host_checks,
+                    int32_t wait_spins);
 
 /* ---- Two-level preconditioner (no counterpart in the reference) -------------------
  * A coarse space of rigid-body modes: the nodes are grouped into aggregates, and each

@@ -66,6 +66,7 @@ SIGNATURES: dict[str, list] = {
     "psx_csr_dirichlet": [_i64, _p, _p, _p, _i32, _p, _p],
     "psx_tet4_adjoint": [_p, _p, _p, _p, _p, _f64, _f64, _p, _p, _p, _p, _p, _i64, _p, _p],
     "psx_pcg": [_i64, _p, _p, _p, _i32, _p, _p, _f64, _f64, _i32, _i32, _p, _i64, _p, _p],
+    "psx_pcg_limited": [_i64, _p, _p, _p, _i32, _p, _p, _f64, _f64, _i32, _i32, _p, _i64, _p, _p, _i32, _i32],
     "psx_pcg_enqueue": [_i64, _p, _p, _p, _i32, _p, _p, _f64, _f64, _i32, _i32, _p, _i64, _p, _p],
     "psx_segment_sumsq": [_i64, _p, _p, _p, _p],
     "psx_fbar_plan_count": [_i64, _p, _p, _p, _p],

@@ -45,6 +45,7 @@ from psierra_b200._lib import check, lib, ptr
 from psierra_b200.assembler import GPUAssembler, raise_if_wait_gave_up
 from psierra_b200.material import NeoHookeanField
 from psierra_b200.meshgen import concat_meshes
+from psierra_b200.solver import raise_if_cg_gave_up
 
 
 def _stream() -> int:
@@ -191,6 +192,7 @@ class BatchedNewton:
             check(lib().psx_pcg_work_bytes(n, self.precond, ctypes.byref(nb)), "psx_pcg_work_bytes")
         self.pcg_work = torch.empty(int(nb.value), dtype=torch.uint8, device=dev)
         self.pcg_status = torch.zeros((int(lib().psx_status_bytes()) + 3) // 4, dtype=torch.int32, device=dev)
+        self.pcg_wait_spins = 0  # polls of one bounded wait of the CG (0 = a second or two)
         self._graph: torch.cuda.CUDAGraph | None = None
 
     # ------------------------------------------------------------------ one iteration
@@ -228,10 +230,10 @@ class BatchedNewton:
                                        self.coarse.struct_ptr(), ptr(self.pcg_work), self.pcg_work.numel(),
                                        ptr(self.pcg_status), _stream(), 0), "psx_pcg_coarse")
         else:
-            check(lib().psx_pcg_enqueue(self.n, ptr(d["indptr"]), ptr(d["indices"]), ptr(self.k), vp, ptr(self.rhs),
+            check(lib().psx_pcg_limited(self.n, ptr(d["indptr"]), ptr(d["indices"]), ptr(self.k), vp, ptr(self.rhs),
                                         ptr(self.du), self.pcg_rtol, 0.0, self.pcg_iterations, self.precond,
-                                        ptr(self.pcg_work), self.pcg_work.numel(), ptr(self.pcg_status), _stream()),
-                  "psx_pcg_enqueue")
+                                        ptr(self.pcg_work), self.pcg_work.numel(), ptr(self.pcg_status), _stream(),
+                                        0, self.pcg_wait_spins), "psx_pcg_limited")
         self.du.mul_(self.scale)
         self.u.add_(self.du)
 
@@ -312,6 +314,8 @@ class BatchedNewton:
                 # the replay assembled with check_status=False: a bounded wait that gave
                 # up leaves a K_T summed out of order, so no instance may use this step
                 raise_if_wait_gave_up(self.asm.status_counts()[3])
+                if not self.per_instance_cg and self.coarse is None:
+                    raise_if_cg_gave_up(self.pcg_status[5].item())  # nor a solution that is no solution
                 hist.append(rn)
                 active = alive & ~conv
                 with np.errstate(invalid="ignore"):

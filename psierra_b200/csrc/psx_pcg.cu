@@ -554,12 +554,13 @@ int layout(int64_t n, int precond, void* work, PcgWork* w, int64_t* bytes) {
 template <typename VT, bool BLOCK, bool NODAL>
 int run_pcg(int64_t n, const int32_t* indptr, const int32_t* indices, const VT* vals, const double* b, double* x,
             double rtol, double atol, int32_t maxiter, const PcgWork& w, Status* st, cudaStream_t s,
-            int identity, bool host_checks) {
+            int identity, bool host_checks, int32_t spins) {
   const int grid_vec = (int)std::min<int64_t>(kGridMax, (n + kBlock - 1) / kBlock);
   const int grid_row = NODAL ? (int)std::min<int64_t>(kGridMax, (n / 3 + kBlock / kNodeLanes - 1) / (kBlock / kNodeLanes))
                              : (int)std::min<int64_t>(kGridMax, (n + kBlock / kRowLanes - 1) / (kBlock / kRowLanes));
   // systems whose state fits the shared memory of the GPU run in one launch
-  const int one = run_pcg_resident<VT, BLOCK, NODAL>(n, indptr, indices, vals, b, x, rtol, atol, maxiter, w, st, s, identity);
+  const int one = run_pcg_resident<VT, BLOCK, NODAL>(n, indptr, indices, vals, b, x, rtol, atol, maxiter, w, st, s, identity,
+                                                     spins);
   if (one != 0) return one > 0 ? PSX_OK : PSX_ERR_CUDA;
   if (cudaMemsetAsync(w.s, 0, sizeof(PcgScalars), s) != cudaSuccess) return PSX_ERR_CUDA;
   if (BLOCK)
@@ -843,7 +844,7 @@ extern "C" int psx_pcg_work_bytes(int64_t n, int precond, int64_t* bytes) {
 namespace {
 int pcg_entry(int64_t n, const int32_t* indptr, const int32_t* indices, const void* values, int value_precision,
               const double* b, double* x, double rtol, double atol, int32_t maxiter, int precond, void* work,
-              int64_t work_bytes, void* status, void* stream, bool host_checks) {
+              int64_t work_bytes, void* status, void* stream, bool host_checks, int32_t spins = 0) {
   using namespace psx;
   if (n <= 0 || !indptr || !indices || !values || !b || !x || !work || !status || maxiter < 0) return PSX_ERR_ARG;
   const bool nodal = (precond & PSX_PCG_NODAL) != 0;
@@ -863,7 +864,7 @@ int pcg_entry(int64_t n, const int32_t* indptr, const int32_t* indices, const vo
   const int id = precond == PSX_PRECOND_NONE;
 #define PSX_RUN(VT, BLK, NOD) \
   run_pcg<VT, BLK, NOD>(n, indptr, indices, static_cast<const VT*>(values), b, x, rtol, atol, maxiter, w, st, s, id, \
-                        host_checks)
+                        host_checks, spins)
   if (value_precision == PSX_FP64) {
     if (nodal) return blk ? PSX_RUN(double, true, true) : PSX_RUN(double, false, true);
     return blk ? PSX_RUN(double, true, false) : PSX_RUN(double, false, false);
@@ -980,6 +981,15 @@ extern "C" int psx_pcg_enqueue(int64_t n, const int32_t* indptr, const int32_t* 
                                void* stream) {
   return pcg_entry(n, indptr, indices, values, value_precision, b, x, rtol, atol, maxiter, precond, work, work_bytes,
                    status, stream, false);
+}
+
+extern "C" int psx_pcg_limited(int64_t n, const int32_t* indptr, const int32_t* indices, const void* values,
+                               int value_precision, const double* b, double* x, double rtol, double atol,
+                               int32_t maxiter, int precond, void* work, int64_t work_bytes, void* status,
+                               void* stream, int host_checks, int32_t wait_spins) {
+  if (wait_spins < 0) return PSX_ERR_ARG;
+  return pcg_entry(n, indptr, indices, values, value_precision, b, x, rtol, atol, maxiter, precond, work, work_bytes,
+                   status, stream, host_checks != 0, wait_spins);
 }
 
 // ---------------------------------------------------------------------------------------

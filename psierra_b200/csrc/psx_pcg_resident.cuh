@@ -12,7 +12,8 @@
 //   Blocks of one thread-block cluster (16, on small systems) meet by the cluster barrier
 // and post into each other's shared memory; more blocks (a cooperative launch, so all are
 // resident) count their arrivals in global memory.  Polls are bounded: a block that gives up
-// reports a breakdown and ends.
+// ends without arriving again, so the others' next meeting gives up too, and block 0 sets status
+// flag bit 0.
 // Measured (block-Jacobi, FP32 values), us per iteration, three launches -> one:
 //   2,187 unknowns 20 -> 5.5, 6,591 21.2 -> 8.5, 46,875 25.6 -> 9.8, 206,763 44.4 -> 18.5.
 // What bounds it: small systems, the meetings; 207,000 unknowns, the product's loads.
@@ -29,7 +30,7 @@ constexpr int kResClusterMax = 16;
 // the time, its product runs on 16 SMs (us per iteration, cluster and grid: 2,187 rows 5.5 and
 // 8.4, 6,591 rows 9.2 and 8.5, 17,496 rows 13.1 and 8.7).
 constexpr int64_t kResClusterRows = 6144;
-constexpr int32_t kResSpins = 1 << 21;     // polls of one meeting: a second or two
+constexpr int32_t kResSpins = 1 << 21;     // default polls of one meeting: a second or two
 
 // What the blocks of the grid form meet on: a count of arrivals, and the sums that each
 // block posts before it arrives, in two sets in turn (a block can be one meeting ahead).
@@ -57,6 +58,7 @@ struct Meeting {
   double (*all)[kResClusterMax][3];  // 2 x 16 x 3 in shared memory (cluster form)
   double (*warp)[3];            // 32 x 3: a block's warps
   double (*eight)[3];           // 8 x 3: the first warps' sums of what the blocks posted
+  int32_t limit;                // polls of one meeting
   unsigned int epoch;
 
   // Every thread's v summed over all threads of all blocks; false when a wait gave up.
@@ -119,7 +121,7 @@ struct Meeting {
         res_arrive(&board->arrived);
         const unsigned int want = epoch * gridDim.x;
         for (int32_t spins = 0; (int)(res_arrived(&board->arrived) - want) < 0;)
-          if (++spins > kResSpins) {
+          if (++spins > limit) {
             gave_up = true;
             break;
           }
@@ -161,7 +163,7 @@ struct ResArgs {
   ResBoard* board;
   Status* st;
   double rtol, atol;
-  int32_t maxiter, identity;
+  int32_t maxiter, identity, spins;
 };
 
 // Matrix values and columns, each read once per product: not kept in L1, which is p's.
@@ -202,7 +204,7 @@ __global__ void __launch_bounds__(res_threads<CLUSTER>(), 1) pcg_resident(ResArg
   }
   const int64_t u0 = (int64_t)blockIdx.x * cap;
   const int own = (int)max((int64_t)0, min((int64_t)cap, A.units - u0));
-  Meeting<CLUSTER> meet{A.board, s_all, s_warp, s_eight, 0};
+  Meeting<CLUSTER> meet{A.board, s_all, s_warp, s_eight, A.spins, 0};
 
   // p of an own unit to global memory, where the neighbours read it
   auto publish = [&](int k, const double* from) {
@@ -309,7 +311,17 @@ __global__ void __launch_bounds__(res_threads<CLUSTER>(), 1) pcg_resident(ResArg
     publish(k, s_x);
   }
   double v[3] = {0.0, 0.0, 0.0};
-  bool ok = meet.template sum<0>(v);
+  auto report = [&](int32_t iters, int32_t flags, double rr) {
+    if (blockIdx.x == 0 && tid == 0) {
+      A.st->iters = iters;
+      A.st->flags = flags;
+      A.st->value = sqrt(rr);
+    }
+  };
+  if (!meet.template sum<0>(v)) {
+    report(0, 1, 0.0);
+    return;
+  }
   product();
   __syncthreads();
   v[0] = v[1] = v[2] = 0.0;
@@ -330,7 +342,7 @@ __global__ void __launch_bounds__(res_threads<CLUSTER>(), 1) pcg_resident(ResArg
       v[1] += r[d] * z[d];
     }
   }
-  ok = meet.template sum<3>(v) && ok;
+  bool ok = meet.template sum<3>(v);
   double rr = v[0], rho = v[1], rho_prev = 0.0;
   const double tol = fmax(A.atol, A.rtol * sqrt(v[2])), tol2 = tol * tol;
   bool converged = v[2] == 0.0 || sqrt(rr) < tol;
@@ -393,11 +405,7 @@ __global__ void __launch_bounds__(res_threads<CLUSTER>(), 1) pcg_resident(ResArg
   for (int k = tid; k < own; k += kThreads)
 #pragma unroll
     for (int d = 0; d < kD; ++d) A.x[kD * (u0 + k) + d] = s_x[d * cap + k];
-  if (blockIdx.x == 0 && tid == 0) {
-    A.st->iters = iters;
-    A.st->flags = ok && converged ? 0 : (ok && breakdown == 2 ? 2 : 4);
-    A.st->value = sqrt(rr);
-  }
+  report(iters, !ok ? 1 : converged ? 0 : breakdown == 2 ? 2 : 4, rr);
 }
 
 // Units per block and blocks of a system, or 0 when its state does not fit the GPU's shared
@@ -457,7 +465,7 @@ inline int res_cluster_blocks(K* kernel, int dev, unsigned long long* known) {
 template <typename VT, bool BLOCK, bool NODAL>
 int run_pcg_resident(int64_t n, const int32_t* indptr, const int32_t* indices, const VT* vals, const double* b, double* x,
                      double rtol, double atol, int32_t maxiter, const PcgWork& w, Status* st, cudaStream_t s,
-                     int identity) {
+                     int identity, int32_t spins) {
   constexpr bool kNode = BLOCK || NODAL;
   constexpr int kD = kNode ? 3 : 1, kDoubles = 4 * kD + (BLOCK ? 9 : kD) + (NODAL ? 1 : 0);
   const int64_t units = n / kD;
@@ -466,7 +474,7 @@ int run_pcg_resident(int64_t n, const int32_t* indptr, const int32_t* indices, c
     return -1;
   if (sms > 256) sms = 256;
   ResArgs A{n, units, 0, indptr, indices, vals, b, x, w.z, reinterpret_cast<ResBoard*>(w.partial), st, rtol, atol, maxiter,
-            identity};
+            identity, spins > 0 ? spins : kResSpins};
   // one cluster on small systems, else one block per SM
   static unsigned long long s_grid = 0, s_cluster = 0;
   const int64_t rows = units * kD;

@@ -45,6 +45,16 @@ class DirectSolver(SparseLinearSolver):
         return spla.spsolve(A, b)
 
 
+WAIT_GAVE_UP = 1  # status flag bit 0: a bounded wait of the one-launch CG gave up
+
+
+def raise_if_cg_gave_up(flags: int) -> None:
+    """Raise when the status ``flags`` of a solve say that a bounded wait gave up: the kernel ran
+    to its end, but its solution is invalid.  Not a breakdown: the matrix is not at fault."""
+    if int(flags) & WAIT_GAVE_UP:
+        raise RuntimeError("psierra_b200: a bounded wait in the CG kernel gave up; the solution is invalid")
+
+
 class PCGResult:
     def __init__(self, iterations: int, converged: bool, residual_norm: float, flags: int):
         self.iterations, self.converged, self.residual_norm, self.flags = iterations, converged, residual_norm, flags
@@ -89,8 +99,16 @@ class ConjugateGradientSolver(SparseLinearSolver):
         self.atol = atol
         self.device = torch.device(device if device is not None else "cuda")
         self.last: PCGResult | None = None
+        self.wait_spins = 0  # polls of one bounded wait in the one-launch form (0 = a second or two)
         self._status = None
         self._work: torch.Tensor | None = None
+
+    def set_wait_limit(self, spins: int) -> None:
+        """Polls after which a bounded wait of the one-launch CG gives up (0 = the default, a
+        second or two); ``solve_device`` and ``solve`` then raise."""
+        if int(spins) < 0:
+            raise ValueError("spins must be >= 0")
+        self.wait_spins = int(spins)
 
     def _workspace(self, n: int, precond: int) -> torch.Tensor:
         nbytes = ctypes.c_int64()
@@ -130,13 +148,15 @@ class ConjugateGradientSolver(SparseLinearSolver):
                                        coarse.struct_ptr(), ptr(work), work.numel(), ptr(self._status),
                                        torch.cuda.current_stream().cuda_stream, 1), "psx_pcg_coarse")
         else:
-            check(lib().psx_pcg(n, ptr(indptr), ptr(indices), ptr(values), vp, ptr(b), ptr(x), float(self.tolerance),
-                                float(self.atol), int(self.max_iterations), precond, ptr(work), work.numel(),
-                                ptr(self._status), torch.cuda.current_stream().cuda_stream), "psx_pcg")
+            check(lib().psx_pcg_limited(n, ptr(indptr), ptr(indices), ptr(values), vp, ptr(b), ptr(x),
+                                        float(self.tolerance), float(self.atol), int(self.max_iterations), precond,
+                                        ptr(work), work.numel(), ptr(self._status),
+                                        torch.cuda.current_stream().cuda_stream, 1, self.wait_spins), "psx_pcg_limited")
         st = self._status.cpu()
         iters, flags = int(st[4]), int(st[5])
         rn = float(st.view(torch.float64)[3])
         self.last = PCGResult(iters, flags == 0, rn, flags)
+        raise_if_cg_gave_up(flags)
         return self.last
 
     def solve(self, A, b) -> np.ndarray:
