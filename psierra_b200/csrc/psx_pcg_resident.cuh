@@ -461,7 +461,9 @@ inline int res_cluster_blocks(K* kernel, int dev, unsigned long long* known) {
   return found;
 }
 
-// 1: solved here; 0: not this system (too large); -1: a CUDA error.
+// 1: solved here; 0: not this system (too large, or the launch is refused, as a cooperative one is
+// where the process has a part of the SMs); -1: a CUDA error.  A refusal's error is cleared and the
+// next form tried; an error of earlier work stays, and the next form's own checks report it.
 template <typename VT, bool BLOCK, bool NODAL>
 int run_pcg_resident(int64_t n, const int32_t* indptr, const int32_t* indices, const VT* vals, const double* b, double* x,
                      double rtol, double atol, int32_t maxiter, const PcgWork& w, Status* st, cudaStream_t s,
@@ -482,24 +484,25 @@ int run_pcg_resident(int64_t n, const int32_t* indptr, const int32_t* indices, c
     auto* kernel = pcg_resident<VT, BLOCK, NODAL, true>;
     const int blocks = res_cluster_blocks(kernel, dev, &s_cluster);
     const ResShape c = res_shape(units, kDoubles, blocks > 0 ? blocks : 1);
-    if (blocks < 0) return -1;
     if (blocks > 0 && c.per_block > 0) {
       A.per_block = c.per_block;
       cudaLaunchAttribute at[1];
       cudaLaunchConfig_t cfg{};
       res_cluster_config(&cfg, at, blocks, c.smem, s);
-      return cudaLaunchKernelEx(&cfg, kernel, A) == cudaSuccess ? 1 : -1;
+      if (cudaLaunchKernelEx(&cfg, kernel, A) == cudaSuccess) return 1;
     }
+    if (blocks != 0) cudaGetLastError();
   }
   const ResShape g = res_shape(units, kDoubles, sms);
   if (g.blocks <= 0) return 0;
   auto* kernel = pcg_resident<VT, BLOCK, NODAL, false>;
-  if (set_dynamic_smem_once(kernel, kResSmem, &s_grid) != cudaSuccess) return -1;
   A.per_block = g.per_block;
-  if (cudaMemsetAsync(A.board, 0, sizeof(unsigned int), s) != cudaSuccess) return -1;
   void* args[] = {&A};
-  return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kernel), dim3(g.blocks), dim3(res_threads<false>()), args, g.smem,
-                                     s) == cudaSuccess
-             ? 1
-             : -1;
+  if (cudaMemsetAsync(A.board, 0, sizeof(unsigned int), s) != cudaSuccess) return -1;
+  if (set_dynamic_smem_once(kernel, kResSmem, &s_grid) == cudaSuccess &&
+      cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kernel), dim3(g.blocks), dim3(res_threads<false>()), args, g.smem,
+                                  s) == cudaSuccess)
+    return 1;
+  cudaGetLastError();
+  return 0;
 }

@@ -1,0 +1,101 @@
+"""One-launch CG solves that the device refuses (GPU): the next form solves them.
+
+A small library in front of libcudart (LD_PRELOAD, in a child process) answers chosen calls with
+an error code and passes every other call on, so nothing that is refused runs.
+"""
+from __future__ import annotations
+
+import os
+import subprocess
+import sys
+import textwrap
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+FRONT = r"""
+#include <cuda_runtime_api.h>
+#include <dlfcn.h>
+extern "C" {
+int front_refuse = 0;   // bit 0: cooperative launches, bit 1: cluster launches
+int front_refused = 0;  // how many were
+int front_grid = 0;     // blocks of the last cluster launch
+int front_narrow = 0;   // the n-th kernel asked for its clusters has none of 16 blocks
+static cudaError_t pending = cudaSuccess;
+static void* real(const char* name) {
+  static void* h = dlopen("libcudart.so.12", RTLD_LAZY | RTLD_NOLOAD);
+  return dlsym(h, name);
+}
+static cudaError_t refuse() { ++front_refused; return pending = cudaErrorCooperativeLaunchTooLarge; }
+cudaError_t cudaLaunchCooperativeKernel(const void* f, dim3 g, dim3 b, void** a, size_t m, cudaStream_t s) {
+  if (front_refuse & 1) return refuse();
+  return ((cudaError_t(*)(const void*, dim3, dim3, void**, size_t, cudaStream_t))real("cudaLaunchCooperativeKernel"))(f, g, b, a, m, s);
+}
+cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* f, void** a) {
+  if (c->numAttrs == 1 && c->attrs[0].id == cudaLaunchAttributeClusterDimension) {
+    if (front_refuse & 2) return refuse();
+    front_grid = c->gridDim.x;
+  }
+  return ((cudaError_t(*)(const cudaLaunchConfig_t*, const void*, void**))real("cudaLaunchKernelExC"))(c, f, a);
+}
+cudaError_t cudaOccupancyMaxActiveClusters(int* n, const void* f, const cudaLaunchConfig_t* c) {
+  static const void* asked[64];
+  int k = 0;
+  while (k < 63 && asked[k] && asked[k] != f) ++k;
+  asked[k] = f;
+  if (k + 1 == front_narrow && c->gridDim.x == 16) { *n = 0; return cudaSuccess; }
+  return ((cudaError_t(*)(int*, const void*, const cudaLaunchConfig_t*))real("cudaOccupancyMaxActiveClusters"))(n, f, c);
+}
+cudaError_t cudaGetLastError(void) {
+  cudaError_t e = pending;
+  pending = cudaSuccess;
+  return e != cudaSuccess ? e : ((cudaError_t(*)(void))real("cudaGetLastError"))();
+}
+}
+"""
+
+CHILD = """
+    import ctypes, sys
+    import numpy as np, torch
+    sys.path[:0] = [{root!r}, {root!r} + "/tests"]
+    from test_pcg_resident_gpu import _solve, _system
+    front = ctypes.CDLL({front!r})
+    word = lambda name: ctypes.c_int.in_dll(front, name)
+
+    def solve(n, dtype=np.float64):
+        A, b = _system(n, True, seed=n)
+        A.data = A.data.astype(np.float32).astype(np.float64)
+        x, r = _solve(A, b, "block-jacobi", True, dtype)
+        assert r.converged and r.iterations <= 60
+        assert np.linalg.norm(b - A @ x) <= 1.01e-10 * np.linalg.norm(b)
+        return x
+"""
+
+
+def _child(tmp_path, body):
+    front = tmp_path / "front.so"
+    (tmp_path / "front.cpp").write_text(FRONT)
+    subprocess.run(["g++", "-shared", "-fPIC", "-O1", "-I/usr/local/cuda/include", "-o", str(front),
+                    str(tmp_path / "front.cpp"), "-ldl"], check=True)
+    code = textwrap.dedent(CHILD).format(root=ROOT, front=str(front)) + textwrap.dedent(body)
+    r = subprocess.run([sys.executable, "-c", code], env={**os.environ, "LD_PRELOAD": str(front)}, cwd=ROOT,
+                       capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-2000:]
+
+
+def test_the_next_form_solves_what_is_refused(tmp_path):
+    _child(tmp_path, """
+    for n in (3000, 30000):  # cluster form, grid form
+        want = solve(n)
+        for bits, times in ((1, n > 6144), (2, n <= 6144), (3, 1 + (n <= 6144))):
+            word("front_refuse").value = bits
+            word("front_refused").value = 0
+            x = solve(n)
+            word("front_refuse").value = 0
+            assert word("front_refused").value == times, (n, bits, word("front_refused").value)
+            # two residuals of 1.01e-10 ||b||, condition below 10
+            assert np.linalg.norm(x - want) <= 2.1e-9 * np.linalg.norm(want)
+        assert np.array_equal(solve(n), want)
+    """)
