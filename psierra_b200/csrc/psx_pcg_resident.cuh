@@ -438,12 +438,14 @@ inline void res_cluster_config(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* at,
 }
 
 // Blocks of the cluster form on this device: 16 where such a cluster fits with a block's whole
-// shared memory, else 8, else 0; -1 on a CUDA error.  Asked once per kernel and device.
+// shared memory, else 8, else 0; -1 on a CUDA error.  Asked once per kernel and device: the
+// kernels differ in registers but not in type, so each caller keeps its own answers (1 + blocks,
+// 0 = not asked).
 template <typename K>
-inline int res_cluster_blocks(K* kernel, int dev, unsigned long long* known) {
-  static int s_blocks[64];
-  const unsigned long long bit = 1ull << (dev & 63);
-  if (__atomic_load_n(known, __ATOMIC_ACQUIRE) & bit) return s_blocks[dev & 63];
+inline int res_cluster_blocks(K* kernel, int dev, int answers[64]) {
+  int* answer = answers + (dev & 63);
+  const int known = __atomic_load_n(answer, __ATOMIC_ACQUIRE);
+  if (known) return known - 1;
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
       cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kResSmem) != cudaSuccess)
     return -1;
@@ -456,8 +458,7 @@ inline int res_cluster_blocks(K* kernel, int dev, unsigned long long* known) {
     if (cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) != cudaSuccess) cudaGetLastError();
     else if (clusters > 0) found = blocks;
   }
-  s_blocks[dev & 63] = found;
-  __atomic_fetch_or(known, bit, __ATOMIC_RELEASE);
+  __atomic_store_n(answer, 1 + found, __ATOMIC_RELEASE);
   return found;
 }
 
@@ -478,11 +479,12 @@ int run_pcg_resident(int64_t n, const int32_t* indptr, const int32_t* indices, c
   ResArgs A{n, units, 0, indptr, indices, vals, b, x, w.z, reinterpret_cast<ResBoard*>(w.partial), st, rtol, atol, maxiter,
             identity, spins > 0 ? spins : kResSpins};
   // one cluster on small systems, else one block per SM
-  static unsigned long long s_grid = 0, s_cluster = 0;
+  static unsigned long long s_grid = 0;
+  static int s_cluster[64];
   const int64_t rows = units * kD;
   if (rows <= kResClusterRows) {
     auto* kernel = pcg_resident<VT, BLOCK, NODAL, true>;
-    const int blocks = res_cluster_blocks(kernel, dev, &s_cluster);
+    const int blocks = res_cluster_blocks(kernel, dev, s_cluster);
     const ResShape c = res_shape(units, kDoubles, blocks > 0 ? blocks : 1);
     if (blocks > 0 && c.per_block > 0) {
       A.per_block = c.per_block;

@@ -99,3 +99,12 @@ def test_the_next_form_solves_what_is_refused(tmp_path):
             assert np.linalg.norm(x - want) <= 2.1e-9 * np.linalg.norm(want)
         assert np.array_equal(solve(n), want)
     """)
+
+
+def test_each_kernel_keeps_its_own_cluster_size(tmp_path):
+    _child(tmp_path, """
+    word("front_narrow").value = 2  # the second kernel, FP32 values, gets 8 blocks
+    for dtype, blocks in ((np.float64, 16), (np.float32, 8), (np.float64, 16), (np.float32, 8)):
+        solve(3000, dtype)
+        assert word("front_grid").value == blocks, (dtype, word("front_grid").value)
+    """)
