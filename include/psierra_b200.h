@@ -566,9 +566,9 @@ int psx_csr_dirichlet(int64_t n, const int32_t* indptr, const int32_t* indices, 
  * default) at the first call that uses the module on that device, which a
  * psx_pcg_static call does.  A caller that must have all its device memory reserved
  * before its run either sets CUDA_MODULE_LOADING=EAGER or makes one psx_pcg_static call
- * on each device during its set-up; later calls reserve nothing more.  The first call on
- * a device also looks up the scratch address on that device; make that first call before
- * any stream capture.  Like psx_pcg, a system that one launch does not take has its
+ * on each device during its set-up; later calls, of any size and with any options, reserve
+ * nothing more.  The first call on a device looks up the scratch address on that device and
+ * loads the kernels of every form; make that first call before any stream capture.  Like psx_pcg, a system that one launch does not take has its
  * convergence test read back to the host every 16 iterations (a device-to-host copy and a
  * synchronisation of `stream`).
  * Every call on a device shares the one array, so calls that overlap on the GPU (other

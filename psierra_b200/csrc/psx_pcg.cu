@@ -1113,6 +1113,31 @@ constexpr int kMaxDevices = 64;
 void* g_pcg_scratch_addr[kMaxDevices] = {};
 std::mutex g_pcg_scratch_mu;
 
+// Load the kernels of every form of psx_pcg (under lazy loading a kernel takes device memory at
+// its first use): the sizes and options of later calls must not reserve any.
+template <typename... K>
+bool load_kernels(K*... kernels) {
+  cudaFuncAttributes at;
+  return (... && (cudaFuncGetAttributes(&at, reinterpret_cast<const void*>(kernels)) == cudaSuccess));
+}
+template <typename VT, bool BLOCK, bool NODAL>
+bool load_forms() {
+  using namespace psx;
+  return load_kernels(pcg_resident<VT, BLOCK, NODAL, true>, pcg_resident<VT, BLOCK, NODAL, false>,
+                      pcg_init_residual<VT, BLOCK, NODAL>, pcg_spmv<VT, NODAL>);
+}
+template <typename VT>
+bool load_forms() {
+  return load_forms<VT, true, true>() && load_forms<VT, true, false>() && load_forms<VT, false, true>() &&
+         load_forms<VT, false, false>();
+}
+bool load_pcg() {
+  using namespace psx;
+  return load_forms<double>() && load_forms<float>() &&
+         load_kernels(jacobi_setup, bjacobi_setup, pcg_init_dots<true>, pcg_init_dots<false>, pcg_update_p<true>,
+                      pcg_update_p<false>, pcg_update_xr<true>, pcg_update_xr<false>, pcg_report);
+}
+
 // Device address of the scratch array on the current device, looked up once per device
 // with that device current (the host-side symbol is only a stand-in, not an address).
 int static_scratch(void** out) {
@@ -1122,7 +1147,7 @@ int static_scratch(void** out) {
   std::lock_guard<std::mutex> lock(g_pcg_scratch_mu);
   if (!g_pcg_scratch_addr[dev]) {
     void* p = nullptr;
-    if (cudaGetSymbolAddress(&p, g_pcg_scratch) != cudaSuccess || !p) return PSX_ERR_CUDA;
+    if (cudaGetSymbolAddress(&p, g_pcg_scratch) != cudaSuccess || !p || !load_pcg()) return PSX_ERR_CUDA;
     g_pcg_scratch_addr[dev] = p;
   }
   *out = g_pcg_scratch_addr[dev];
