@@ -56,10 +56,14 @@ def _time(asm, u, precision, want_f, want_k, f, k, reps: int) -> float:
 
 
 def _apply(asm, want_k: bool, lag: int, bps: int, slack: int, split: bool | None = None) -> None:
+    """Queue the sweeps tuned, in this shape; the others stay queued or in two passes as they are."""
+    other_queued = getattr(asm.pattern, "queued_f" if want_k else "queued_k", True)
     if want_k:
         asm.set_queue(lag=lag, blocks_per_sm=bps, ring_slack=slack, split=split)
     else:
         asm.set_queue(lag_f=lag, blocks_per_sm=bps, ring_slack=slack)
+    if not other_queued:  # the blocks per SM queue them too
+        asm.set_two_pass(f=want_k, k=not want_k)
 
 
 def tune(asm, u: torch.Tensor, precision: str | None = None, want_f: bool = True, want_k: bool = True,

@@ -53,8 +53,9 @@ class MeshPattern:
         self._dev: dict | None = None
         self._blocks: tuple | None = None
         self._plan_host: dict | None = None
-        self.queued_f = False  # a lag of the f / K.v queue was chosen (set_queue)
-        self.queued_k = False  # a lag of the K queue or one of its kernels was chosen
+        # shapes of a queue chosen through set_queue: its lag, its kernel, or the blocks per SM of both
+        self.queued_f = False  # f / K.v queue
+        self.queued_k = False  # K queue
         self.granule, self.tile, self.tile_items, self.lag, self.lag_f, self.ring_slack = self.QUEUE[npe]
         self.blocks_per_sm = 0
         self.wait_spins = 0  # polls of one bounded wait in the persistent kernels (0 = about a second)
@@ -244,8 +245,8 @@ class MeshPattern:
 
     @property
     def two_pass(self) -> bool:
-        """Whether the sweeps without a tangent run in two passes: by default, until a lag of
-        their queue is chosen (``set_queue(lag_f=...)``) or its waits are limited."""
+        """Whether the sweeps without a tangent run in two passes: by default, until a shape of
+        their queue is chosen (``set_queue(lag_f=..., blocks_per_sm=...)``) or its waits are limited."""
         return not self.queued_f and self.wait_spins == 0
 
     # Elements up to which tangent sweeps run in two passes too.  Tet4, FP32 (above
@@ -260,8 +261,8 @@ class MeshPattern:
     @property
     def two_pass_k(self) -> bool:
         """The same for the tangent sweeps (Tet10, and FP32 ones of Tet4) of meshes up to
-        ``TWO_PASS_K_ELEMENTS``: until a lag of the K queue or one of its kernels
-        (``set_queue(lag=..., split=...)``) is chosen."""
+        ``TWO_PASS_K_ELEMENTS``: until a shape of the K queue or one of its kernels
+        (``set_queue(lag=..., split=..., blocks_per_sm=...)``) is chosen."""
         return not self.queued_k and self.wait_spins == 0 and self.n_elements <= self.TWO_PASS_K_ELEMENTS
 
     # Largest mesh (elements) on point records, and where they start in FP32.  At the upper end
@@ -312,7 +313,9 @@ class MeshPattern:
         warp-specialised kernel (``split``; the mixed kernel otherwise).
 
         With ``lag_f``, the sweeps without a tangent run the queued kernel instead of two
-        passes; with ``lag`` or ``split``, the tangent sweeps too (``set_two_pass`` goes back).
+        passes; with ``lag`` or ``split``, the tangent sweeps; with ``blocks_per_sm`` other than
+        0, both, as two passes fill the GPU (``set_two_pass`` goes back).  ``ring_slack`` alone
+        chooses nothing: two passes have no ring.
         Rebuilds the task queues when a lag changes; a workspace sized for the old values must
         be re-queried (``psx_work_bytes``) afterwards.
         """
@@ -327,6 +330,8 @@ class MeshPattern:
             self.queued_f = True
         if blocks_per_sm is not None:
             self.blocks_per_sm = int(blocks_per_sm)
+            if self.blocks_per_sm > 0:
+                self.queued_f = self.queued_k = True
         if ring_slack is not None:
             self.ring_slack = int(ring_slack)
         if split is not None:
