@@ -34,9 +34,14 @@ DEFAULT_SPLITS = (True, False)
 _cache: dict[str, tuple] = {}
 
 
+# What was compared.  An entry of an earlier set does not say which of today's ways is the fastest
+# (before the two launches every entry named a queue), so it is not used: the mesh is timed again.
+_WAYS = "queue,two-pass"
+
+
 def _key(asm, precision: str, want_f: bool, want_k: bool) -> str:
     name = torch.cuda.get_device_name(asm.device)
-    return f"{name}|npe{asm.npe}|E{asm.n_elements}|N{asm.n_nodes}|{precision}|f{int(want_f)}k{int(want_k)}"
+    return f"{name}|npe{asm.npe}|E{asm.n_elements}|N{asm.n_nodes}|{precision}|f{int(want_f)}k{int(want_k)}|{_WAYS}"
 
 
 def _time(asm, u, precision, want_f, want_k, f, k, reps: int) -> float:
@@ -85,9 +90,8 @@ def tune(asm, u: torch.Tensor, precision: str | None = None, want_f: bool = True
             disk = json.load(fh)
     hit = _cache.get(key) or (tuple(disk[key]) if key in disk else None)
     if hit is not None:
-        hit = tuple(hit) + (asm.pattern.split,) * (4 - len(hit))
         _apply(asm, want_k, *hit[:4])
-        if len(hit) > 4 and hit[4]:
+        if hit[4]:
             asm.set_two_pass(f=not want_k, k=want_k)
         return {"lag": hit[0], "blocks_per_sm": hit[1], "ring_slack": hit[2], "split": hit[3], "ms": None,
                 "table": {}}
@@ -103,16 +107,16 @@ def tune(asm, u: torch.Tensor, precision: str | None = None, want_f: bool = True
                     _apply(asm, want_k, lag, bps, slack, split)
                     table[(lag, bps, slack, split)] = _time(asm, u, prec, want_f, want_k, f, k, reps)
     best = min(table, key=table.get)
-    entry = best
+    two_pass = False
     _apply(asm, want_k, *best)
     if hasattr(asm, "set_two_pass"):
         # sweeps that also run in two passes, without a queue: keep the faster way
         asm.set_two_pass(f=not want_k, k=want_k)
-        if (asm.pattern.tangent_in_two_passes(prec) if want_k else asm.pattern.two_pass) and \
-                _time(asm, u, prec, want_f, want_k, f, k, reps) < table[best]:
-            entry = best + (True,)
-        else:
+        two_pass = bool(asm.pattern.tangent_in_two_passes(prec) if want_k else asm.pattern.two_pass) and \
+            _time(asm, u, prec, want_f, want_k, f, k, reps) < table[best]
+        if not two_pass:
             _apply(asm, want_k, *best)
+    entry = best + (two_pass,)
     _cache[key] = entry
     if cache_file:
         disk[key] = list(entry)
