@@ -71,16 +71,24 @@ def _apply(asm, want_k: bool, lag: int, bps: int, slack: int, split: bool | None
         asm.set_two_pass(f=want_k, k=not want_k)
 
 
+def _result(entry: tuple, ms: float | None, table: dict) -> dict:
+    return dict(zip(("lag", "blocks_per_sm", "ring_slack", "split", "two_pass"), entry), ms=ms, table=table)
+
+
 def tune(asm, u: torch.Tensor, precision: str | None = None, want_f: bool = True, want_k: bool = True,
          lags=DEFAULT_LAGS, blocks=DEFAULT_BLOCKS, slacks=DEFAULT_SLACKS, splits=DEFAULT_SPLITS, reps: int = 5,
          cache_file: str | None = None) -> dict:
-    """Pick (lag, blocks_per_sm, ring_slack, split) for ``asm`` by timing; applies and returns it.
+    """Pick the queue's (lag, blocks_per_sm, ring_slack, split) or two passes for ``asm`` by timing;
+    applies and returns the choice.
 
     The lag tuned is that of the queue the sweep uses (the K queue when ``want_k``, else
     the f queue).  ``splits`` is swept only for Tet4 FP32 tangent sweeps (the only ones
     with a warp-specialised kernel); elsewhere split is left as it is.  Returns
-    ``{"lag", "blocks_per_sm", "ring_slack", "split", "ms", "table": {(lag, bps, slack,
-    split): ms}}``.  With a cached entry for the same key nothing is timed.
+    ``{"two_pass", "ms", "lag", "blocks_per_sm", "ring_slack", "split", "table": {(lag, bps, slack,
+    split): ms}}``: whether two passes won, the time of what runs now, the best queue and the
+    queues' times.  With a cached entry for the same key nothing is timed (``ms`` is None).
+
+    A tangent's queue holds for both precisions of the pattern, as its lag does.
     """
     prec = precision or asm.precision
     key = _key(asm, prec, want_f, want_k)
@@ -93,8 +101,7 @@ def tune(asm, u: torch.Tensor, precision: str | None = None, want_f: bool = True
         _apply(asm, want_k, *hit[:4])
         if hit[4]:
             asm.set_two_pass(f=not want_k, k=want_k)
-        return {"lag": hit[0], "blocks_per_sm": hit[1], "ring_slack": hit[2], "split": hit[3], "ms": None,
-                "table": {}}
+        return _result(hit, None, {})
     f = asm.new_f() if want_f else None
     k = asm.new_k(prec) if want_k else None
     has_split = asm.npe == 4 and want_k and prec == "fp32-mixed"
@@ -107,13 +114,14 @@ def tune(asm, u: torch.Tensor, precision: str | None = None, want_f: bool = True
                     _apply(asm, want_k, lag, bps, slack, split)
                     table[(lag, bps, slack, split)] = _time(asm, u, prec, want_f, want_k, f, k, reps)
     best = min(table, key=table.get)
-    two_pass = False
+    two_pass, ms = False, table[best]
     _apply(asm, want_k, *best)
     if hasattr(asm, "set_two_pass"):
         # sweeps that also run in two passes, without a queue: keep the faster way
         asm.set_two_pass(f=not want_k, k=want_k)
-        two_pass = bool(asm.pattern.tangent_in_two_passes(prec) if want_k else asm.pattern.two_pass) and \
-            _time(asm, u, prec, want_f, want_k, f, k, reps) < table[best]
+        if asm.pattern.tangent_in_two_passes(prec) if want_k else asm.pattern.two_pass:
+            passes_ms = _time(asm, u, prec, want_f, want_k, f, k, reps)
+            two_pass, ms = passes_ms < ms, min(passes_ms, ms)
         if not two_pass:
             _apply(asm, want_k, *best)
     entry = best + (two_pass,)
@@ -122,5 +130,4 @@ def tune(asm, u: torch.Tensor, precision: str | None = None, want_f: bool = True
         disk[key] = list(entry)
         with open(cache_file, "w") as fh:
             json.dump(disk, fh, indent=1, sort_keys=True)
-    return {"lag": best[0], "blocks_per_sm": best[1], "ring_slack": best[2], "split": best[3], "ms": table[best],
-            "table": table}
+    return _result(entry, ms, table)

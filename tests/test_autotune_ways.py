@@ -68,11 +68,13 @@ def test_the_faster_way_is_kept_and_replayed(tune, tmp_path, ms, way, want_k):
     cache = str(tmp_path / "tune.json")
     asm, r, timed = tune(ms, want_k, cache_file=cache)
     assert asm.way == way and timed[-1] == ("two-pass",) and len(timed) == 3
+    assert r["two_pass"] == (way == ("two-pass",)) and r["ms"] == min(ms, 1.0)  # what runs, and its time
     for forget in (False, True):  # from memory, from the file
         if forget:
             autotune._cache.clear()
         asm, r, timed = tune(99.0, want_k, cache_file=cache)
         assert asm.way == way and timed == [] and r["lag"] == 16
+        assert r["two_pass"] == (way == ("two-pass",)) and r["ms"] is None
 
 
 def test_entries_of_one_way_are_timed_again(tune, tmp_path):
