@@ -46,6 +46,20 @@ NCU_CAPTURE_ELEMENTS = 1053696
 NCU_TRAFFIC = {"fk32": 292.361216e6 + 174.428928e6, "kv32": 87.758336e6 + 2.580736e6}
 
 
+def fk_sweep(plan, split: bool) -> tuple[str, bool]:
+    """The kernels of the FP32-mixed f+K sweep of a plan, and whether NCU_TRAFFIC is theirs."""
+    if plan.two_pass_p & 2:
+        return ("tet4_points_kernel<float> F|K (element factors), then tet4_point_items_kernel<float> (blocks formed and "
+                "summed, one thread per node pair and node)"), True
+    if plan.two_pass_k:
+        return ("tet4_tiles_kernel<float> F|K (element tiles, one warp each), then tet4_items_kernel (tile records summed, "
+                "one thread per node pair and node)"), False
+    if split:
+        return ("tet4_split_kernel<float> F|K (per SM 8 element-tile warps + 8 owner-computes gather warps, registers "
+                "moved between them by setmaxnreg)"), False
+    return "tet4_persistent_kernel<float> F|K (element tiles + owner-computes gather in the same warps)", False
+
+
 def parse():
     ap = argparse.ArgumentParser()
     ap.add_argument("--gpus", type=int, default=1)
@@ -629,11 +643,7 @@ def main():
         from psierra_b200 import _lib
 
         split = asm.pattern.split and _lib.lib().psx_tet4_split_ready() == 1
-        fk_kernel = ("tet4_points_kernel<float> F|K (element factors), then tet4_point_items_kernel<float> (blocks "
-                     "formed and summed, one thread per node pair and node)" if asm.dev["plan"].two_pass_p & 2 else
-                     "tet4_split_kernel<float> F|K (per SM 8 element-tile warps + 8 owner-computes gather warps, "
-                     "registers moved between them by setmaxnreg)" if split else
-                     "tet4_persistent_kernel<float> F|K (element tiles + owner-computes gather in the same warps)")
+        fk_kernel, fk_captured = fk_sweep(asm.dev["plan"], split)
         line = {
             "metric": METRIC, "value": world * E / (ms_mixed * 1e-3), "unit": "elements/s", "n_gpus": world,
             "steps": args.steps, "warmup": args.warmup, "ms_per_step": ms_mixed, "higher_is_better": True,
@@ -645,9 +655,10 @@ def main():
                               "K.v: 512 MB L2 flush before every timed step"),
                        "parallelism": f"replicas x{world}" if world > 1 else "single GPU"},
             "roofline": {"bound": "hbm", "achieved": ach, "peak": peak, "unit": "GB/s", "frac": ach / peak,
-                         "traffic": NCU_TRAFFIC["fk32"] * E / NCU_CAPTURE_ELEMENTS,
+                         "traffic": NCU_TRAFFIC["fk32"] * E / NCU_CAPTURE_ELEMENTS if fk_captured else None,
                          "traffic_note": "bytes per sweep: ncu DRAM read+write of the cube 56^3 sweep's two launches scaled by "
-                                         "elements (latency-bound: DRAM throughput 30% and 34% in that capture)",
+                                         "elements (latency-bound: DRAM throughput 30% and 34% in that capture)"
+                                         if fk_captured else "no capture of the kernels of this mesh size",
                          "peak_kind": peak_kind,
                          "algorithmic_bytes_per_launch": bytes_mixed, "kernel": fk_kernel,
                          "launches_per_step": asm.launches_per_call("fp32-mixed")},
