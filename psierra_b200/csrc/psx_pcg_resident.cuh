@@ -58,7 +58,7 @@ struct Meeting {
   double (*all)[kResClusterMax][3];  // 2 x 16 x 3 in shared memory (cluster form)
   double (*warp)[3];            // 32 x 3: a block's warps
   double (*eight)[3];           // 8 x 3: the first warps' sums of what the blocks posted
-  int32_t limit;                // polls of one meeting
+  const int32_t& limit;         // polls of one meeting, in the kernel's parameters
   unsigned int epoch;
 
   // Every thread's v summed over all threads of all blocks; false when a wait gave up.
@@ -183,8 +183,11 @@ __device__ __forceinline__ int32_t res_once(const int32_t* p) {
   return v;
 }
 
+// The arguments stay in the parameter space: with the poll limit in one of the grid form's 64
+// registers an iteration of 206,763 unknowns takes 19.1 us, read from there 18.8 (18.7 with a
+// constant limit).
 template <typename VT, bool BLOCK, bool NODAL, bool CLUSTER>
-__global__ void __launch_bounds__(res_threads<CLUSTER>(), 1) pcg_resident(ResArgs A) {
+__global__ void __launch_bounds__(res_threads<CLUSTER>(), 1) pcg_resident(const __grid_constant__ ResArgs A) {
   constexpr int kThreads = res_threads<CLUSTER>();
   constexpr bool kNode = BLOCK || NODAL;  // a unit is a node (three rows) or a row
   constexpr int kD = kNode ? 3 : 1;
