@@ -430,9 +430,9 @@ int psx_pcg_work_bytes(int64_t n, int precond, int64_t* bytes);
  * iters = iterations, flags = 0 converged / 2 max iterations reached / 4 breakdown / 1 a
  * bounded wait of the one-launch form gave up (x is then invalid),
  * value = final ||r||.  Dot products are reduced in a fixed order (bitwise
- * reproducible).  A system whose state fits the GPU's shared memory (176 bytes per node with
- * block-Jacobi and nodal rows: about 578,000 unknowns) is solved in one launch, without host
- * reads; above that the call synchronises the stream every 16 iterations to test convergence.
+ * reproducible).  A system whose state fits the GPU's shared memory beside a useful L1 (176 bytes per
+ * node with block-Jacobi and nodal rows: about 500,000 unknowns) is solved in one launch, without
+ * host reads; above that the call synchronises the stream every 16 iterations to test convergence.
  */
 int psx_pcg(int64_t n, const int32_t* indptr, const int32_t* indices, const void* values,
             int value_precision, const double* b, double* x, double rtol, double atol, int32_t maxiter,

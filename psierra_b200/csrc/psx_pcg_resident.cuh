@@ -24,7 +24,13 @@
 template <bool CLUSTER>
 constexpr int res_threads() { return CLUSTER ? 512 : 1024; }
 constexpr int kResLanes = 8;               // lanes per node / row of the product, as in spmv_node
-constexpr int kResSmem = 224 * 1024;       // state of a block's own nodes
+// State of a block's own nodes.  With it the block takes up to 196 KB of the SM's memory (960 bytes
+// of its own and 1 KB of the system's besides), which leaves the gathers of p 60 KB of L1.  The next
+// carve-out, 228 KB, leaves 28, and the neighbours' p no longer stay: Kuhn cubes, block-Jacobi and
+// nodal rows, us per iteration, one launch / three: 499,125 unknowns (193 KB) FP32 50 / 60, FP64
+// 67 / 99; 526,848 (204 KB) 81 / 63 and 118 / 101.  Jacobi, rows: 714,984 (189 KB) FP64 114 / 127,
+// 750,141 (198 KB) 197 / 135.
+constexpr int kResSmem = 194 * 1024;
 constexpr int kResClusterMax = 16;
 // Rows up to which one cluster is faster than a block per SM: its meetings take a third of
 // the time, its product runs on 16 SMs (us per iteration, cluster and grid: 2,187 rows 5.5 and

@@ -21,6 +21,7 @@ FRONT = r"""
 extern "C" {
 int front_refuse = 0;   // bit 0: cooperative launches, bit 1: cluster launches
 int front_refused = 0;  // how many were
+int front_coop = 0;     // cooperative launches
 int front_grid = 0;     // blocks of the last cluster launch
 int front_narrow = 0;   // the n-th kernel asked for its clusters has none of 16 blocks
 static cudaError_t pending = cudaSuccess;
@@ -31,6 +32,7 @@ static void* real(const char* name) {
 static cudaError_t refuse() { ++front_refused; return pending = cudaErrorCooperativeLaunchTooLarge; }
 cudaError_t cudaLaunchCooperativeKernel(const void* f, dim3 g, dim3 b, void** a, size_t m, cudaStream_t s) {
   if (front_refuse & 1) return refuse();
+  ++front_coop;
   return ((cudaError_t(*)(const void*, dim3, dim3, void**, size_t, cudaStream_t))real("cudaLaunchCooperativeKernel"))(f, g, b, a, m, s);
 }
 cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* f, void** a) {
@@ -107,4 +109,26 @@ def test_each_kernel_keeps_its_own_cluster_size(tmp_path):
     for dtype, blocks in ((np.float64, 16), (np.float32, 8), (np.float64, 16), (np.float32, 8)):
         solve(3000, dtype)
         assert word("front_grid").value == blocks, (dtype, word("front_grid").value)
+    """)
+
+
+@pytest.mark.parametrize("precond,unit", [("block-jacobi", 176), ("jacobi", 128)])
+def test_large_systems_leave_the_gathers_their_cache(tmp_path, precond, unit):
+    # one block per SM, 194 KB of state: the last system that one launch takes and the next one
+    _child(tmp_path, f"""
+    from psierra_b200.solver import ConjugateGradientSolver
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    last = 3 * sms * (194 * 1024 // {unit})
+    for n, launches in ((last, 1), (last + 3, 0)):
+        # 3 x 3 blocks 4 I and nothing else: solved in one iteration
+        t = lambda a, d: torch.from_numpy(np.ascontiguousarray(a, dtype=d)).cuda()
+        rows = np.arange(n)
+        indices = 3 * (rows // 3)[:, None] + np.arange(3)
+        values = 4.0 * (indices == rows[:, None])
+        b, x = torch.ones(n, dtype=torch.float64, device="cuda"), torch.zeros(n, dtype=torch.float64, device="cuda")
+        word("front_coop").value = 0
+        r = ConjugateGradientSolver(tolerance=1e-10, preconditioner="{precond}").solve_device(
+            t(3 * np.arange(n + 1), np.int32), t(indices, np.int32), t(values, np.float64), b, x, nodal=True)
+        assert r.converged and torch.equal(x, 0.25 * b)
+        assert word("front_coop").value == launches, (n, word("front_coop").value)
     """)
