@@ -1105,15 +1105,16 @@ extern "C" int psx_point_lists(const psx_plan_t* plan, void* stream) {
 }
 
 extern "C" int psx_work_bytes(const psx_plan_t* plan, int precision, int64_t* ring_elems, int64_t* bytes) {
-  // one workspace serves both task queues: the larger of their layouts
-  psx::WorkLayout Wk, Wf;
-  int rc = psx::work_layout(plan, precision, nullptr, &Wk, 3, true);
-  if (rc != PSX_OK) return rc;
-  rc = psx::work_layout(plan, precision, nullptr, &Wf, 3, false);
-  if (rc != PSX_OK) return rc;
-  if (!ring_elems || !bytes) return PSX_ERR_ARG;
-  *ring_elems = Wk.ring_elems > Wf.ring_elems ? Wk.ring_elems : Wf.ring_elems;
-  *bytes = Wk.total_bytes > Wf.total_bytes ? Wk.total_bytes : Wf.total_bytes;
+  // one workspace serves every sweep: the largest of their layouts
+  if (!plan || !ring_elems || !bytes) return PSX_ERR_ARG;
+  *ring_elems = *bytes = 0;
+  for (int i = 0; i < (plan->npe == 4 ? 3 : 2); ++i) {  // f, K, and the linear and mass matrices of Tet4
+    psx::WorkLayout W;
+    const int rc = psx::work_layout(plan, precision, nullptr, &W, 3, i > 0, i == 2);
+    if (rc != PSX_OK) return rc;
+    *ring_elems = std::max(*ring_elems, W.ring_elems);
+    *bytes = std::max(*bytes, W.total_bytes);
+  }
   return PSX_OK;
 }
 
@@ -1131,7 +1132,7 @@ extern "C" int psx_tet4_assemble(const psx_plan_t* plan, const double* X, const 
   if (wantF && !f_out) return PSX_ERR_ARG;
   if (wantK && !k_out) return PSX_ERR_ARG;
   WorkLayout W;
-  int rc = work_layout(plan, precision, work, &W, kMinBlocks, wantK || linear);
+  int rc = work_layout(plan, precision, work, &W, kMinBlocks, wantK || linear, linear);
   if (rc != PSX_OK) return rc;
   if (work_bytes < W.total_bytes) return PSX_ERR_ARG;
   Tet4Args A{plan->conn, X, u, nullptr, nullptr, nullptr, mu_e, kappa_e, mu, kappa, lam, static_cast<Status*>(status)};
