@@ -181,7 +181,7 @@ __device__ __forceinline__ void tet4_element(const Tet4Args& A, int64_t e, const
       tet4_sums<KT>(tc, p, q, gk, Vn, S);
       double yr[12];
       if constexpr (kAdj)
-        tet4_vjp(A, e, true, ps, l, G, Un, Vn, tc, S, yr);
+        tet4_vjp(A, e, ps, l, G, Un, Vn, tc, S, yr);
       else
         tet4_product<KT>(tc, p, q, gk, S, yr);
       store_f12<FGLOBAL>(frec, yr);
@@ -1001,7 +1001,7 @@ int run_tet4(const psx_plan_t* P, const Tet4Args& A, const WorkLayout& W, KT* k_
     if (P->two_pass) return run_two_pass<KT, MODE>(P, A, W, nullptr, f_out, stream, dr);
   }
   if constexpr (kWantK && sizeof(KT) == 8 && (MODE & (PSX_LINEAR | PSX_MASS | kModeEff)) == 0) {
-    if ((P->two_pass_p & (sizeof(KT) == 8 ? 1 : 2))) return run_points<KT, MODE>(P, A, W, k_out, f_out, stream);
+    if (P->two_pass_p & 1) return run_points<KT, MODE>(P, A, W, k_out, f_out, stream);
   }
   const GatherArgs g = gather_args(P, W.ring_elems);
   const QueueArgs Q = queue_args(P, W, kWantK);

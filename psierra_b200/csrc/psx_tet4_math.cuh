@@ -195,9 +195,9 @@ __device__ __forceinline__ void tet4_product(const TangentCoef<KT>& tc, const KT
 
 // Vector-Jacobian product of w.f_e with f_e,a = V P g_a (the adjoint of
 // tet4_total_lagrangian.py:136-137 w.r.t. X, mu, kappa): the coordinates' part into yr, the
-// moduli's into A.dmu[e], A.dkappa[e] when `params`.  L_w = sum_b w_b g_b^T,
+// moduli's into A.dmu[e], A.dkappa[e].  L_w = sum_b w_b g_b^T,
 // VM = V dP/dF[L_w] = alpha F^-T + hb Pv F^-T + beta c F + phi Gv^T.
-__device__ __forceinline__ void tet4_vjp(const Tet4Args& A, int64_t e, bool params, const PointState& ps,
+__device__ __forceinline__ void tet4_vjp(const Tet4Args& A, int64_t e, const PointState& ps,
                                          const double l[3][3], const Tet4Geom& G, const double Un[4][3],
                                          const double Vn[4][3], const TangentCoef<double>& tc,
                                          const Tet4Sums<double>& S, double yr[12]) {
@@ -264,7 +264,7 @@ __device__ __forceinline__ void tet4_vjp(const Tet4Args& A, int64_t e, bool para
     for (int j = 0; j < 3; ++j) yr[3 * (j + 1) + i] = Z[i][j];
   }
   // parameter gradients: dP/dmu = 2 J^-2/3 F^-T dev E, dP/dkappa = ln J F^-T
-  if (params && (A.dmu || A.dkappa)) {
+  if (A.dmu || A.dkappa) {
     double E[3][3], trE = 0.0;
 #pragma unroll
     for (int i = 0; i < 3; ++i)
