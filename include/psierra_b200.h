@@ -439,10 +439,11 @@ int psx_pcg(int64_t n, const int32_t* indptr, const int32_t* indices, const void
             int precond, void* work, int64_t work_bytes, void* status, void* stream);
 
 /*
- * psx_pcg with a fixed trip count and no host synchronisation (no counterpart in the
- * reference, whose solves always return to Python): exactly maxiter iterations are
- * enqueued on the stream and become no-ops once converged, so the call can be captured
- * in a CUDA graph.  Same arguments, results and status as psx_pcg.
+ * psx_pcg without host synchronisation (no counterpart in the reference, whose solves always
+ * return to Python), so that the call can be captured in a CUDA graph: one launch that ends
+ * when it has converged or done maxiter iterations, or, for systems that one launch does not
+ * take, exactly maxiter iterations that become no-ops once converged.  Same arguments, results
+ * and status as psx_pcg.
  */
 int psx_pcg_enqueue(int64_t n, const int32_t* indptr, const int32_t* indices, const void* values,
                     int value_precision, const double* b, double* x, double rtol, double atol, int32_t maxiter,

@@ -19,8 +19,8 @@
 //
 // Kernels (one thread per element, node, one-ring entry or two-ring block; every sum in a
 // fixed order, the reference's ascending element / patch node but for the longest lists,
-// which a warp adds as a tree).  Measured on 162,000 elements, us (before): 11 (16), 9 (9),
-// 30 (51), 54 (122), 111 (154), 59 (96).  What bounds them: the volumetric pass its
+// which a warp adds as a tree).  Measured on 162,000 elements, us, in the order below: 11,
+// 9, 30, 54, 111, 59.  What bounds them: the volumetric pass its
 // instructions and gathered loads, the element pass 12 warps per SM and its 134 MB of records,
 // the gather the latency of their loads.
 //   fbar_pre     V_e, J_e, q_e (and the inversion status)

@@ -9,6 +9,8 @@
 // with the Jacobi preconditioner of the reference (1/diag where |diag| > 1e-14, else 1)
 // or a 3x3 block-Jacobi preconditioner (inverse of each node's diagonal block).
 //
+// Systems whose state fits the SMs' shared memory beside a useful L1 run in one launch
+// (psx_pcg_resident.cuh); the rest, and launches that the device refuses, as follows.
 // Three kernels per iteration: p-update, SpMV (+ p.q), and the fused x/r/z update
 // (+ r.r, r.z).  Every dot product is reduced deterministically: each block reduces its
 // share with a fixed tree and stores a partial; the last block to finish (atomic

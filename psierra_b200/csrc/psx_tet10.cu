@@ -370,7 +370,7 @@ tet10_persistent_kernel(Tet10Args A, GatherArgs g, QueueArgs Q, KT* __restrict__
 // per pair / node.  The queue kept every SM at 8 warps (252 registers) for both phases and
 // its gathers, latency bound, waited on element tiles; split, a tile takes 168 registers and
 // no task (12 warps per SM), and the gathers run at their own occupancy with cached 32-byte
-// loads.  Kuhn cubes, us, one launch before / two passes: f + K FP64 384 elements 35 / 23,
+// loads.  Kuhn cubes, us, queue / two passes: f + K FP64 384 elements 35 / 23,
 // 10,368 79 / 56, 162,000 1035 / 685, 750,000 4041 / 3280; FP32 162,000 652 / 493; f 384
 // elements 16 / 11, 162,000 200 / 76.  Tiles: 8 warps per SM 730 us (FP64 f + K, batches of
 // 2), 9 and more 708.  Pass 1 is bound by shared memory and FP64 latency, pass 2 by DRAM

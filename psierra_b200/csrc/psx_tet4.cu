@@ -582,12 +582,12 @@ tet4_split_kernel(Tet4Args A, GatherArgs g, QueueArgs Q, const int4* __restrict_
 // that hold only what an element tile needs, and gathers at full occupancy instead of a turn
 // in the queue.  The records of the whole mesh are kept (22 bytes per element without a
 // tangent, in L2 up to about 5M elements; 141 with one: psierra_b200/pattern.py has the
-// lines).  Measured, queue -> two passes, us:
+// lines, and the tangents' times).  Measured, queue -> two passes, us:
 //   elements    f              K.v FP32        K.v FP64      f + K FP32
-//     384,000    71 ->  25      69 ->  31       80 ->  33     119 ->  91
-//   1,053,696   106 ->  56     120 ->  68      121 ->  80     237 -> 244 (point records)
-//   3,072,000   272 -> 146     297 -> 181      320 -> 220     639 -> 672 (point records)
-// What bounds them now: without a tangent the latency of the FP64 element chain (the FP64
+//     384,000    71 ->  25      69 ->  31       80 ->  33     119 ->  93
+//   1,053,696   106 ->  56     120 ->  68      121 ->  80     238 -> 243
+//   3,072,000   272 -> 146     297 -> 181      320 -> 220     637 -> 668
+// What bounds them: without a tangent the latency of the FP64 element chain (the FP64
 // pipe alone would take 21 us at 1.05M elements); with one, half each, pass 1 at 12 warps per
 // SM (shared memory of the staged blocks) and the scattered record reads and 12-byte row
 // segments of pass 2.  Passing over the mesh in pieces only adds launches (f, 1.05M elements,
@@ -751,10 +751,10 @@ __global__ void tet4_dets_kernel(const int32_t* __restrict__ conn, const double*
 // (22 bytes per element), the FP64 ones are stored per element, as the queue sums them.
 // Measured on Kuhn cubes, us, f + K (K):
 //   elements    FP64 queue     points         FP32 queue / tiles   points
-//     384,000    203 (185)     118 (107)         94  (84)           80  (68)
-//   1,053,696    520 (476)     283 (241)        235 (219)          180 (152)
-//   3,072,000   1564 (1420)    775 (691)        634 (584)          485 (405)
-// Pass 1 takes 179 of the last 485 us (FP64 chain at 20 warps per SM, 45% of issue slots),
+//     384,000    203 (185)     118 (107)         93  (83)           78  (64)
+//   1,053,696    520 (476)     283 (241)        238 (222)          180 (153)
+//   3,072,000   1564 (1420)    775 (691)        637 (584)          481 (410)
+// Pass 1 takes 179 of the last 481 us (FP64 chain at 20 warps per SM, 45% of issue slots),
 // pass 2 the rest: gathered 32-byte loads (62M sectors through L1, 1.0 GB of DRAM traffic,
 // 3.1 TB/s).  What made the difference there: node blocks spread among the pair blocks, so
 // that both read a record while it is in L2 (1.05M elements, FP64: 377 -> 317 us); planes
@@ -996,7 +996,8 @@ int run_tet4(const psx_plan_t* P, const Tet4Args& A, const WorkLayout& W, KT* k_
              cudaStream_t stream, const DRArgs& dr = DRArgs{}) {
   constexpr bool kWantK =
       (MODE & (PSX_WANT_K | PSX_LINEAR | PSX_MASS)) != 0 && (MODE & (PSX_KV | kModeAdjoint)) == 0;
-  // every sweep without a tangent is faster in two passes (tet4_tiles_kernel), at all sizes
+  // every sweep without a tangent is faster in two passes (tet4_tiles_kernel), at all sizes: the
+  // queue runs it where its shape or a limit on its waits is asked for
   if constexpr (!kWantK) {
     if (P->two_pass) return run_two_pass<KT, MODE>(P, A, W, nullptr, f_out, stream, dr);
   }

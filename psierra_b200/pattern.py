@@ -252,10 +252,12 @@ class MeshPattern:
     # Elements up to which tangent sweeps run in two passes too.  Tet4, FP32 (above
     # POINT_ELEMENTS_FP32 the effective tangent alone): their records (141 bytes per element) then
     # stay in L2 between the passes; f + K on Kuhn cubes, us, two passes / queue: 82,944 elements
-    # 27 / 42, 196,608 47 / 85, 384,000 91 / 119, 663,552 159 / 209, 1,053,696 234 / 235,
-    # 3,072,000 652 / 630.  Tet10: two passes stay ahead (750,000 elements, FP64, 3280 / 4000
+    # 26 / 42, 196,608 46 / 84, 384,000 93 / 119, 663,552 155 / 213, 1,053,696 243 / 238,
+    # 3,072,000 668 / 637 (effective tangent 253 / 251 and 696 / 674).  Tet10: two passes stay ahead (750,000 elements, FP64, 3280 / 4000
     # us), but their records (5.2 KB per element) grow with the mesh, here to 4.1 GB; the
-    # queue's ring does not.
+    # queue's ring does not.  Sweeps without a tangent have no such line: their records (22 bytes
+    # per Tet4 element, 240 per Tet10) end with the mesh sizes, 0.7 GB at the 2^25 elements of
+    # one Tet4 mesh, 1.4 GB where a Tet10 mesh reaches nnz 2^31.
     TWO_PASS_K_ELEMENTS = 3 << 18
 
     @property
@@ -266,10 +268,11 @@ class MeshPattern:
         return not self.queued_k and self.wait_spins == 0 and self.n_elements <= self.TWO_PASS_K_ELEMENTS
 
     # Largest mesh (elements) on point records, and where they start in FP32.  At the upper end
-    # they hold 3.0 GB (FP64); the queue's ring does not grow with the mesh.  f + K on Kuhn
-    # cubes, us, points / queue (FP64) or the shorter of queue and two passes (FP32): FP64 384
+    # they hold 3.0 GB (FP64); the queue's ring does not grow with the mesh.  The lists that they
+    # need (48 bytes per element) are built with every plan up to there.  f + K on Kuhn cubes, us, points / queue (FP64) or the shorter of queue and two passes (FP32): FP64 384
     # elements 13 / 18, 48,000 26 / 42, 384,000 112 / 202, 3,072,000 775 / 1564, same bits; FP32
-    # 48,000 18 / 15, 162,000 34 / 34, 235,824 47 / 51, 384,000 73 / 89, 3,072,000 480 / 634.
+    # 48,000 18 / 15, 82,944 27 / 26, 196,608 45 / 46, 384,000 78 / 93, 663,552 123 / 155,
+    # 1,053,696 180 / 238, 3,072,000 481 / 637.
     # FP32 sums are associated differently there, so one mesh's bits depend on its schedule.
     POINT_ELEMENTS = 1 << 23
     POINT_ELEMENTS_FP32 = 1 << 18
