@@ -119,9 +119,10 @@ class GPUAssembler:
 
     def workspace(self, precision: str) -> torch.Tensor:
         layout = self.dev["layout"]
-        if layout != self._work_layout:
+        if layout is not self._work_layout:
             # the pattern's queue or passes were chosen anew, by this assembler or another one
-            self._work.clear()
+            if layout != self._work_layout:
+                self._work.clear()
             self._work_layout = layout
         w = self._work.get(precision)
         if w is None:
